@@ -251,8 +251,9 @@ void pmi::fill_args(pm_request *r) {
     for (int k = 0; k < r->S; ++k) {
         float M[9], c[3];
         compose(r->R[0], r->t[0], r->R[k + 1], r->t[k + 1], M, c);
-        for (int row = 0; row < 3; ++row)
-            a.P.G[k][row] = make_float4(M[3 * row], M[3 * row + 1], M[3 * row + 2], c[row]);
+        a.P.G[k][0] = make_float4(M[0], M[3], M[1], M[4]);
+        a.P.G[k][1] = make_float4(M[2], M[5], c[0], c[1]);
+        a.P.G[k][2] = make_float4(M[6], M[7], M[8], c[2]);
         a.src.quad[k] = r->quad[k];
         a.src.tex[k] = (unsigned long long)r->tex[k];
     }

@@ -50,9 +50,8 @@ __device__ __forceinline__ float2 box_muller(uint32_t a, uint32_t b) {
 // ---------------------------------------------------------------------------
 // atan on [0, 1]: atan(t) ~ t * P(t^2), P of degree 7, a minimax (Remez
 // exchange) fit made for this project (max error 3.7e-8 rad before float
-// rounding).  The two coefficient sets below are that polynomial scaled to
-// turns (1/2pi, longitude) and half turns (1/pi, latitude) so the angles come
-// out directly in image-fraction units.
+// rounding).  sample_coords scales it to turns (1/2pi), so the angles come out
+// directly in image-fraction units.
 // ---------------------------------------------------------------------------
 #define PM_ATAN_C0 0.9999993443489075f
 #define PM_ATAN_C1 -0.33329859375953674f
@@ -63,17 +62,43 @@ __device__ __forceinline__ float2 box_muller(uint32_t a, uint32_t b) {
 #define PM_ATAN_C6 0.021862957626581192f
 #define PM_ATAN_C7 -0.004054567310959101f
 
-template <int kScaleInvPi>  // 1: scale by 1/pi; 2: scale by 1/(2 pi)
-__device__ __forceinline__ float atan_poly_scaled(float x2) {
-    constexpr float s = kScaleInvPi == 1 ? 0.318309886183790671538f : 0.159154943091895335769f;
-    float p = PM_ATAN_C7 * s;
-    p = fmaf(p, x2, PM_ATAN_C6 * s);
-    p = fmaf(p, x2, PM_ATAN_C5 * s);
-    p = fmaf(p, x2, PM_ATAN_C4 * s);
-    p = fmaf(p, x2, PM_ATAN_C3 * s);
-    p = fmaf(p, x2, PM_ATAN_C2 * s);
-    p = fmaf(p, x2, PM_ATAN_C1 * s);
-    return fmaf(p, x2, PM_ATAN_C0 * s);
+// Packed FP32 pairs (fma.rn.f32x2 and friends): two independent IEEE
+// operations per instruction, each rounded exactly as its scalar form.  A pair
+// occupies both FMA pipes for the two cycles that two scalar operations take,
+// but one issue slot instead of two, and the sample loop was bound by issue
+// slots: 72.6 -> 55 warp instructions per sample with the rotation, the two
+// angle polynomials and the moments in pairs (1920x960, 6 sources, 8 sweeps:
+// 61.3 -> 58.0 ms; 3840x1920, 8 FP16 sources: 389 -> 373 ms; maps
+// bit-identical).  What binds now is the FMA pipes and their register reads:
+// three register pairs as operands take three cycles instead of two, which is
+// why the last step of the coordinates is scalar, with the scale a constant
+// (69 against 71 cycles per sample in a loop of the cost alone).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ f32x2 pack2(float2 v) { return pack2(v.x, v.y); }
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 
 // Both angles use atan2(a, b) = pi/4 + atan((a - b) / (a + b)) for a, b >= 0,
@@ -83,31 +108,45 @@ __device__ __forceinline__ float atan_poly_scaled(float x2) {
 // coordinates stay in [0, W] x [0, H], which the quad samplers index without
 // further checks (texture reads clamp in hardware and skip the two clamps).
 
-// atan2(x, z) / (2 pi) in [-1/2, 1/2]: the equirectangular longitude of
-// direction (x, ., z) as a fraction of the image width (PatchMatchCuda.cu:140,143).
-// x = z = 0 gives t = -1 and an angle of 0, like atan2(0, 0).
+// Sample coordinates (u, v) of direction (X, Y, Z), as a pair:
+//   u = W lon + halfW, lon = atan2(X, Z) / (2 pi) in [-1/2, 1/2], the
+//       equirectangular longitude in image widths (PatchMatchCuda.cu:140,143);
+//       X = Z = 0 gives t = -1 and an angle of 0, like atan2(0, 0);
+//   v = H lat + halfH, lat = asin(Y / |(X, Y, Z)|) / pi in [-1/2, 1/2], minus
+//       the latitude in image heights (PatchMatchCuda.cu:139,144), evaluated
+//       as atan2(|Y|, sqrt(X^2 + Z^2)) with the sign of Y.
+// The two polynomials run as one pair in units of turns; a half turn is 2
+// turns exactly, so scale = (W, 2 H) gives v the same bits as a latitude
+// polynomial in half turns.  The result's halves are adjacent registers, as
+// the texture fetch reads them.
 template <bool kBound>
-__device__ __forceinline__ float lon_turns(float x, float z) {
-    const float ax = fabsf(x), az = fabsf(z) + 1e-30f;
-    const float t = __fdividef(ax - az, ax + az);
-    float a = fmaf(atan_poly_scaled<2>(t * t), t, 0.125f);
-    if (kBound) a = fmaxf(a, 0.0f);
-    a = (z < 0.0f) ? 0.5f - a : a;
-    return copysignf(a, x);
-}
-
-// asin(y / |(x, y, z)|) / pi in [-1/2, 1/2]: minus the equirectangular
-// latitude as a fraction of the image height (PatchMatchCuda.cu:139,144),
-// evaluated as atan2(|y|, sqrt(x^2 + z^2)) with the sign of y.
-template <bool kBound>
-__device__ __forceinline__ float lat_halfturns(float x, float y, float z) {
-    const float r2 = fmaxf(fmaf(x, x, z * z), 1e-30f);
+__device__ __forceinline__ f32x2 sample_coords(float X, float Y, float Z, f32x2 scale, f32x2 half) {
+    constexpr float s = 0.159154943091895335769f;  // 1 / (2 pi)
+    const float ax = fabsf(X), az = fabsf(Z) + 1e-30f;
+    const float r2 = fmaxf(fmaf(X, X, Z * Z), 1e-30f);
     const float rho = r2 * rsqrtf(r2);
-    const float ay = fabsf(y);
-    const float t = __fdividef(ay - rho, ay + rho);
-    float a = fmaf(atan_poly_scaled<1>(t * t), t, 0.25f);
-    if (kBound) a = fminf(a, 0.5f);
-    return copysignf(a, y);
+    const float ay = fabsf(Y);
+    float rx, ry;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(ax + az));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(ay + rho));
+    const f32x2 t = mul2(pack2(ax - az, ay - rho), pack2(rx, ry));
+    const f32x2 q = mul2(t, t);
+    f32x2 p = pack2(PM_ATAN_C7 * s, PM_ATAN_C7 * s);
+    p = fma2(p, q, pack2(PM_ATAN_C6 * s, PM_ATAN_C6 * s));
+    p = fma2(p, q, pack2(PM_ATAN_C5 * s, PM_ATAN_C5 * s));
+    p = fma2(p, q, pack2(PM_ATAN_C4 * s, PM_ATAN_C4 * s));
+    p = fma2(p, q, pack2(PM_ATAN_C3 * s, PM_ATAN_C3 * s));
+    p = fma2(p, q, pack2(PM_ATAN_C2 * s, PM_ATAN_C2 * s));
+    p = fma2(p, q, pack2(PM_ATAN_C1 * s, PM_ATAN_C1 * s));
+    p = fma2(p, q, pack2(PM_ATAN_C0 * s, PM_ATAN_C0 * s));
+    float2 a = unpack2(fma2(p, t, pack2(0.125f, 0.125f)));
+    if (kBound) {
+        a.x = fmaxf(a.x, 0.0f);
+        a.y = fminf(a.y, 0.25f);
+    }
+    a.x = (Z < 0.0f) ? 0.5f - a.x : a.x;
+    const float2 sc = unpack2(scale), hf = unpack2(half);
+    return pack2(fmaf(copysignf(a.x, X), sc.x, hf.x), fmaf(copysignf(a.y, Y), sc.y, hf.y));
 }
 
 // ---------------------------------------------------------------------------
@@ -133,23 +172,32 @@ struct QuadU8 {
     // shift: value subtracted from every texel, given as 2^23 + I_c so the
     // byte-to-float conversion and the centring are one subtraction.
     static __device__ __forceinline__ float shift_for(float centre) { return 8388608.0f + centre; }
-    static __device__ __forceinline__ float sample(const void *quad, unsigned long long, int qpitch, float u, float v,
-                                                   float shift) {
-        // u in [0, W], v in [0, H] by construction of the angle functions
-        int x0, y0;
+    // Footprint of one sample: the packed texels and the bilinear weights.
+    struct Raw {
+        uint32_t w;
         float ax, ay;
-        split_coord(u, x0, ax);
-        split_coord(v, y0, ay);
-        const uint32_t w = __ldg(static_cast<const uint32_t *>(quad) + (y0 * qpitch + x0));
-        // bytes -> floats minus the centre intensity: (2^23 + byte) - (2^23 + c)
+    };
+    static __device__ __forceinline__ Raw fetch(const void *quad, unsigned long long, int qpitch, float u, float v) {
+        // u in [0, W], v in [0, H] by construction of sample_coords
+        int x0, y0;
+        Raw f;
+        split_coord(u, x0, f.ax);
+        split_coord(v, y0, f.ay);
+        f.w = __ldg(static_cast<const uint32_t *>(quad) + (y0 * qpitch + x0));
+        return f;
+    }
+    static __device__ __forceinline__ float centred(const Raw &f, float shift) {
         // texels as 2^23 + byte; differences are exact, the shift is applied once per row
-        const float m00 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540));
-        const float m01 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541));
-        const float m10 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7542));
-        const float m11 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7543));
-        const float a = fmaf(ax, m01 - m00, m00 - shift);
-        const float b = fmaf(ax, m11 - m10, m10 - shift);
-        return fmaf(ay, b - a, a);
+        const float m00 = __uint_as_float(__byte_perm(f.w, 0x4B000000u, 0x7540));
+        const float m01 = __uint_as_float(__byte_perm(f.w, 0x4B000000u, 0x7541));
+        const float m10 = __uint_as_float(__byte_perm(f.w, 0x4B000000u, 0x7542));
+        const float m11 = __uint_as_float(__byte_perm(f.w, 0x4B000000u, 0x7543));
+        const float a = fmaf(f.ax, m01 - m00, m00 - shift);
+        const float b = fmaf(f.ax, m11 - m10, m10 - shift);
+        return fmaf(f.ay, b - a, a);
+    }
+    static __device__ __forceinline__ f32x2 centred2(const Raw &f, const Raw &g, float shift) {
+        return pack2(centred(f, shift), centred(g, shift));
     }
 };
 
@@ -157,19 +205,28 @@ struct QuadF16 {
     static constexpr float kCoordOffset = 0.0f;
     static constexpr bool kBound = true;
     static __device__ __forceinline__ float shift_for(float centre) { return centre; }
-    static __device__ __forceinline__ float sample(const void *quad, unsigned long long, int qpitch, float u, float v,
-                                                   float shift) {
-        int x0, y0;
+    struct Raw {
+        uint2 w;
         float ax, ay;
-        split_coord(u, x0, ax);
-        split_coord(v, y0, ay);
-        const uint2 w = __ldg(static_cast<const uint2 *>(quad) + (y0 * qpitch + x0));
-        const float2 r0 = __half22float2(*reinterpret_cast<const __half2 *>(&w.x));
-        const float2 r1 = __half22float2(*reinterpret_cast<const __half2 *>(&w.y));
+    };
+    static __device__ __forceinline__ Raw fetch(const void *quad, unsigned long long, int qpitch, float u, float v) {
+        int x0, y0;
+        Raw f;
+        split_coord(u, x0, f.ax);
+        split_coord(v, y0, f.ay);
+        f.w = __ldg(static_cast<const uint2 *>(quad) + (y0 * qpitch + x0));
+        return f;
+    }
+    static __device__ __forceinline__ float centred(const Raw &f, float shift) {
+        const float2 r0 = __half22float2(*reinterpret_cast<const __half2 *>(&f.w.x));
+        const float2 r1 = __half22float2(*reinterpret_cast<const __half2 *>(&f.w.y));
         const float t00 = r0.x - shift, t01 = r0.y - shift, t10 = r1.x - shift, t11 = r1.y - shift;
-        const float a = fmaf(ax, t01 - t00, t00);
-        const float b = fmaf(ax, t11 - t10, t10);
-        return fmaf(ay, b - a, a);
+        const float a = fmaf(f.ax, t01 - t00, t00);
+        const float b = fmaf(f.ax, t11 - t10, t10);
+        return fmaf(f.ay, b - a, a);
+    }
+    static __device__ __forceinline__ f32x2 centred2(const Raw &f, const Raw &g, float shift) {
+        return pack2(centred(f, shift), centred(g, shift));
     }
 };
 
@@ -181,9 +238,13 @@ struct TexU8 {
     static constexpr float kCoordOffset = 0.5f;
     static constexpr bool kBound = false;
     static __device__ __forceinline__ float shift_for(float centre) { return centre; }
-    static __device__ __forceinline__ float sample(const void *, unsigned long long tex, int, float u, float v,
-                                                   float shift) {
-        return fmaf(tex2D<float>((cudaTextureObject_t)tex, u, v), 255.0f, -shift);
+    typedef float Raw;
+    static __device__ __forceinline__ float fetch(const void *, unsigned long long tex, int, float u, float v) {
+        return tex2D<float>((cudaTextureObject_t)tex, u, v);
+    }
+    static __device__ __forceinline__ float centred(float raw, float shift) { return fmaf(raw, 255.0f, -shift); }
+    static __device__ __forceinline__ f32x2 centred2(float f, float g, float shift) {
+        return fma2(pack2(f, g), pack2(255.0f, 255.0f), pack2(-shift, -shift));
     }
 };
 
@@ -191,9 +252,13 @@ struct TexF16 {
     static constexpr float kCoordOffset = 0.5f;
     static constexpr bool kBound = false;
     static __device__ __forceinline__ float shift_for(float centre) { return centre; }
-    static __device__ __forceinline__ float sample(const void *, unsigned long long tex, int, float u, float v,
-                                                   float shift) {
-        return tex2D<float>((cudaTextureObject_t)tex, u, v) - shift;
+    typedef float Raw;
+    static __device__ __forceinline__ float fetch(const void *, unsigned long long tex, int, float u, float v) {
+        return tex2D<float>((cudaTextureObject_t)tex, u, v);
+    }
+    static __device__ __forceinline__ float centred(float raw, float shift) { return raw - shift; }
+    static __device__ __forceinline__ f32x2 centred2(float f, float g, float shift) {
+        return add2(pack2(f, g), pack2(-shift, -shift));
     }
 };
 
@@ -256,6 +321,7 @@ __device__ __forceinline__ void refine_normals4(uint32_t seed, uint32_t kf, uint
 // does not hoist all sources' rows into registers (that spills).
 struct ParamAccess {
     static __device__ __forceinline__ float val(const float &x) { return x; }
+    static __device__ __forceinline__ float2 pair(const float &x) { return make_float2((&x)[0], (&x)[1]); }
     static __device__ __forceinline__ float4 row(const float4 &g) { return g; }
     static __device__ __forceinline__ unsigned long long tex(const unsigned long long &t) { return t; }
     static __device__ __forceinline__ const void *ptr(const void *const &p) { return p; }
@@ -265,6 +331,12 @@ struct SharedAccess {
         float v;
         const unsigned a = (unsigned)__cvta_generic_to_shared(&x);
         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+        return v;
+    }
+    static __device__ __forceinline__ float2 pair(const float &x) {
+        float2 v;
+        const unsigned a = (unsigned)__cvta_generic_to_shared(&x);
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
         return v;
     }
     static __device__ __forceinline__ float4 row(const float4 &g) {
@@ -287,12 +359,22 @@ struct SharedAccess {
     }
 };
 
-// M b for the pose rows g0, g1, g2 (their xyz; w holds c), the
-// hypothesis-independent part of the warp, evaluated directly.
-__device__ __forceinline__ float3 rotate(const float4 &g0, const float4 &g1, const float4 &g2, float bx, float by,
-                                         float bz) {
-    return make_float3(fmaf(g0.x, bx, fmaf(g0.y, by, g0.z * bz)), fmaf(g1.x, bx, fmaf(g1.y, by, g1.z * bz)),
-                       fmaf(g2.x, bx, fmaf(g2.y, by, g2.z * bz)));
+// M b of one source: the first two components as a pair and the third, the
+// hypothesis-independent part of the warp.
+struct Rotated {
+    f32x2 xy;
+    float z;
+};
+
+// M b for a source's pose block, evaluated directly; bx2, by2, bz2 hold each
+// bearing component in both halves.
+__device__ __forceinline__ Rotated rotate(const float4 &g0, const float4 &g1, const float4 &g2, f32x2 bx2, f32x2 by2,
+                                          f32x2 bz2) {
+    const float bx = unpack2(bx2).x, by = unpack2(by2).x, bz = unpack2(bz2).x;
+    Rotated m;
+    m.xy = fma2(pack2(g0.x, g0.y), bx2, fma2(pack2(g0.z, g0.w), by2, mul2(pack2(g1.x, g1.y), bz2)));
+    m.z = fmaf(g2.x, bx, fmaf(g2.y, by, g2.z * bz));
+    return m;
 }
 
 // Factored form over the equirectangular grid: with b = (cos lat sin lon,
@@ -320,11 +402,11 @@ __host__ __device__ constexpr bool factored_warp() {
 }
 __device__ __forceinline__ float3 col_factor(const float4 &g0, const float4 &g1, const float4 &g2, float sin_lon,
                                              float cos_lon) {
-    return make_float3(fmaf(sin_lon, g0.x, cos_lon * g0.z), fmaf(sin_lon, g1.x, cos_lon * g1.z),
+    return make_float3(fmaf(sin_lon, g0.x, cos_lon * g1.x), fmaf(sin_lon, g0.y, cos_lon * g1.y),
                        fmaf(sin_lon, g2.x, cos_lon * g2.z));
 }
 __device__ __forceinline__ float3 row_factor(const float4 &g0, const float4 &g1, const float4 &g2, float sin_lat) {
-    return make_float3(-sin_lat * g0.y, -sin_lat * g1.y, -sin_lat * g2.y);
+    return make_float3(-sin_lat * g0.z, -sin_lat * g0.w, -sin_lat * g2.y);
 }
 
 // x with its sign bit flipped when sg (0 or 0x80000000) is set.
@@ -332,49 +414,76 @@ __device__ __forceinline__ float flip_sign(float x, uint32_t sg) { return __uint
 
 template <int S, class Img, class Acc = ParamAccess>
 struct TapAccum {
-    float swy[S], swyy[S], swxy[S];
+    // moments of sources 2k and 2k + 1 as pairs; an odd last source on its own
+    static constexpr int kPairs = S / 2;
+    f32x2 py[kPairs + 1], pyy[kPairs + 1], pxy[kPairs + 1];
+    float oy, oyy, oxy;
     __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int r = 0; r < S; ++r) swy[r] = swyy[r] = swxy[r] = 0.0f;
+        for (int k = 0; k < kPairs; ++k) py[k] = pyy[k] = pxy[k] = 0ull;
+        oy = oyy = oxy = 0.0f;
     }
+    __device__ __forceinline__ static float part(const f32x2 (&p)[kPairs + 1], float odd, int r) {
+        if (r >= 2 * kPairs) return odd;
+        const float2 v = unpack2(p[r >> 1]);
+        return (r & 1) ? v.y : v.x;
+    }
+    __device__ __forceinline__ float swy(int r) const { return part(py, oy, r); }
+    __device__ __forceinline__ float swyy(int r) const { return part(pyy, oyy, r); }
+    __device__ __forceinline__ float swxy(int r) const { return part(pxy, oxy, r); }
     // One tap given |s| (s = pi . b) and the sources' signed rotated
-    // bearings mb(r) = sign(s) M_r b (a float3): X_r = sign(s) M_r b + |s| c_r.
+    // bearings mb(r) = sign(s) M_r b (a Rotated): X_r = sign(s) M_r b + |s| c_r.
     // P and src live in kernel parameter space (or shared memory, through
-    // Acc); w: bilateral weight, xs: tap intensity minus centre; halfW/halfH
-    // include the sampler's coordinate offset.
+    // Acc); w: bilateral weight, xs: tap intensity minus centre; scale =
+    // (W, 2 H), half = (W / 2, H / 2) plus the sampler's coordinate offset.
     template <class MB>
-    __device__ __forceinline__ void add_rot(const PmPoses &P, const SrcSet &src, float Wf, float Hf, float halfW,
-                                            float halfH, float shift, float as, MB mb, float w, float xs) {
+    __device__ __forceinline__ void add_rot(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half, float shift,
+                                            float as, MB mb, float w, float xs) {
         // phase 1: all S sample coordinates, so the S footprint loads issue
         // back to back; phase 2: bilinear + moments as they arrive
-        float u[S], v[S];
+        f32x2 uv[S];
+        const f32x2 as2 = pack2(as, as);
 #pragma unroll
         for (int r = 0; r < S; ++r) {
-            const float3 m = mb(r);
-            const float X = fmaf(as, Acc::val(P.G[r][0].w), m.x);
-            const float Y = fmaf(as, Acc::val(P.G[r][1].w), m.y);
+            const Rotated m = mb(r);
+            const float2 c = Acc::pair(P.G[r][1].z);
+            const float2 XY = unpack2(fma2(as2, pack2(c), m.xy));
             const float Z = fmaf(as, Acc::val(P.G[r][2].w), m.z);
-            u[r] = fmaf(Wf, lon_turns<Img::kBound>(X, Z), halfW);
-            v[r] = fmaf(Hf, lat_halfturns<Img::kBound>(X, Y, Z), halfH);
+            uv[r] = sample_coords<Img::kBound>(XY.x, XY.y, Z, scale, half);
         }
+        typename Img::Raw raw[S];
 #pragma unroll
         for (int r = 0; r < S; ++r) {
-            const float y = Img::sample(Acc::ptr(src.quad[r]), Acc::tex(src.tex[r]), src.qpitch, u[r], v[r], shift);
+            const float2 c = unpack2(uv[r]);
+            raw[r] = Img::fetch(Acc::ptr(src.quad[r]), Acc::tex(src.tex[r]), src.qpitch, c.x, c.y);
+        }
+        const f32x2 w2 = pack2(w, w), xs2 = pack2(xs, xs);
+#pragma unroll
+        for (int k = 0; k < kPairs; ++k) {
+            const f32x2 y = Img::centred2(raw[2 * k], raw[2 * k + 1], shift);
+            const f32x2 wy = mul2(w2, y);
+            py[k] = add2(py[k], wy);
+            pyy[k] = fma2(wy, y, pyy[k]);
+            pxy[k] = fma2(wy, xs2, pxy[k]);
+        }
+        if constexpr (S & 1) {
+            const float y = Img::centred(raw[S - 1], shift);
             const float wy = w * y;
-            swy[r] += wy;
-            swyy[r] = fmaf(wy, y, swyy[r]);
-            swxy[r] = fmaf(wy, xs, swxy[r]);
+            oy += wy;
+            oyy = fmaf(wy, y, oyy);
+            oxy = fmaf(wy, xs, oxy);
         }
     }
     // One tap with bearing b = (bx, by, bz), rotated per source directly.
-    __device__ __forceinline__ void add_bearing(const PmPoses &P, const SrcSet &src, float Wf, float Hf, float halfW,
-                                                float halfH, float shift, float px, float py, float pz, float bx,
-                                                float by, float bz, float w, float xs) {
-        const float s = fmaf(px, bx, fmaf(py, by, pz * bz));
+    __device__ __forceinline__ void add_bearing(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half,
+                                                float shift, float px, float py_, float pz, float bx, float by,
+                                                float bz, float w, float xs) {
+        const float s = fmaf(px, bx, fmaf(py_, by, pz * bz));
         const uint32_t sg = __float_as_uint(s) & 0x80000000u;
         const float sbx = flip_sign(bx, sg), sby = flip_sign(by, sg), sbz = flip_sign(bz, sg);
-        add_rot(P, src, Wf, Hf, halfW, halfH, shift, fabsf(s),
-                [&](int r) { return rotate(Acc::row(P.G[r][0]), Acc::row(P.G[r][1]), Acc::row(P.G[r][2]), sbx, sby, sbz); },
+        const f32x2 bx2 = pack2(sbx, sbx), by2 = pack2(sby, sby), bz2 = pack2(sbz, sbz);
+        add_rot(P, src, scale, half, shift, fabsf(s),
+                [&](int r) { return rotate(Acc::row(P.G[r][0]), Acc::row(P.G[r][1]), Acc::row(P.G[r][2]), bx2, by2, bz2); },
                 w, xs);
     }
     // One tap at the grid point with row trig rt = (cos lat, sin lat) and
@@ -382,25 +491,24 @@ struct TapAccum {
     // factored_warp<S>() (the arithmetic of the staged tile factors), the
     // direct rotation of the bearing otherwise; the bearing is
     // (cos lat sin lon, -sin lat, cos lat cos lon), as in the staged tile.
-    __device__ __forceinline__ void add_trig(const PmPoses &P, const SrcSet &src, float Wf, float Hf, float halfW,
-                                             float halfH, float shift, float px, float py, float pz, float2 rt,
-                                             float2 ct, float w, float xs) {
+    __device__ __forceinline__ void add_trig(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half, float shift,
+                                             float px, float py_, float pz, float2 rt, float2 ct, float w, float xs) {
         const float bx = rt.x * ct.x, by = -rt.y, bz = rt.x * ct.y;
         if constexpr (factored_warp<S>()) {
-            const float s = fmaf(px, bx, fmaf(py, by, pz * bz));
+            const float s = fmaf(px, bx, fmaf(py_, by, pz * bz));
             const uint32_t sg = __float_as_uint(s) & 0x80000000u;
             const float sc = flip_sign(rt.x, sg);
-            add_rot(P, src, Wf, Hf, halfW, halfH, shift, fabsf(s),
+            add_rot(P, src, scale, half, shift, fabsf(s),
                     [&](int r) {
                         const float4 g0 = Acc::row(P.G[r][0]), g1 = Acc::row(P.G[r][1]), g2 = Acc::row(P.G[r][2]);
                         const float3 A = col_factor(g0, g1, g2, ct.x, ct.y);
                         const float3 B = row_factor(g0, g1, g2, rt.y);
-                        return make_float3(fmaf(sc, A.x, flip_sign(B.x, sg)), fmaf(sc, A.y, flip_sign(B.y, sg)),
-                                           fmaf(sc, A.z, flip_sign(B.z, sg)));
+                        return Rotated{pack2(fmaf(sc, A.x, flip_sign(B.x, sg)), fmaf(sc, A.y, flip_sign(B.y, sg))),
+                                       fmaf(sc, A.z, flip_sign(B.z, sg))};
                     },
                     w, xs);
         } else {
-            add_bearing(P, src, Wf, Hf, halfW, halfH, shift, px, py, pz, bx, by, bz, w, xs);
+            add_bearing(P, src, scale, half, shift, px, py_, pz, bx, by, bz, w, xs);
         }
     }
 };
@@ -478,14 +586,14 @@ template <int S, class Img, class Acc>
 __device__ __forceinline__ void source_nccs(const TapAccum<S, Img, Acc> &acc, float sw, float swx, float swxx, int mode,
                                             float (&sep)[S], float (&cum)[S]) {
 #pragma unroll
-    for (int r = 0; r < S; ++r) sep[r] = ncc_from_moments(sw, swx, swxx, acc.swy[r], acc.swyy[r], acc.swxy[r]);
+    for (int r = 0; r < S; ++r) sep[r] = ncc_from_moments(sw, swx, swxx, acc.swy(r), acc.swyy(r), acc.swxy(r));
     if (mode == PM_COMBINE_FOLD) {
         float cy = 0.f, cyy = 0.f, cxy = 0.f;
 #pragma unroll
         for (int r = 0; r < S; ++r) {
-            cy += acc.swy[r];
-            cyy += acc.swyy[r];
-            cxy += acc.swxy[r];
+            cy += acc.swy(r);
+            cyy += acc.swyy(r);
+            cxy += acc.swxy(r);
             const float n = (float)(r + 1);
             cum[r] = ncc_from_moments(n * sw, n * swx, n * swxx, cy, cyy, cxy);
         }

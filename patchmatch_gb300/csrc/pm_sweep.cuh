@@ -260,8 +260,9 @@ __device__ __forceinline__ void accumulate_plane(TapAccum<S, Img, Acc> &acc, con
                                                  float py, float pz) {
     const int nt = a.patch_half + 1, ph = a.patch_half;
     const float shift = Img::shift_for(Ic);
-    const float halfW = fmaf(0.5f, Acc::val(a.Wf), Img::kCoordOffset);
-    const float halfH = fmaf(0.5f, Acc::val(a.Hf), Img::kCoordOffset);
+    const float Wf = Acc::val(a.Wf), Hf = Acc::val(a.Hf);
+    const f32x2 scale = pack2(Wf, 2.0f * Hf);
+    const f32x2 half = pack2(fmaf(0.5f, Wf, Img::kCoordOffset), fmaf(0.5f, Hf, Img::kCoordOffset));
     acc.zero();
 #pragma unroll 1
     for (int m1 = 0; m1 < nt; ++m1) {
@@ -279,16 +280,15 @@ __device__ __forceinline__ void accumulate_plane(TapAccum<S, Img, Acc> &acc, con
                 const float s = fmaf(px, e.x, fmaf(py, e.y, pz * e.z));
                 const float4 *fa = fac + pa * kTileCols + cbase + m2;
                 const float4 *fb = fac + S * kFactorA + (s < 0.0f ? kTileRows : 0) + tr;
-                acc.add_rot(a.P, a.src, Acc::val(a.Wf), Acc::val(a.Hf), halfW, halfH, shift, fabsf(s),
+                acc.add_rot(a.P, a.src, scale, half, shift, fabsf(s),
                             [&](int r) {
                                 const float4 ca = fa[r * kFactorA], rb = fb[r * kFactorB];
-                                return make_float3(fmaf(rb.w, ca.x, rb.x), fmaf(rb.w, ca.y, rb.y),
-                                                   fmaf(rb.w, ca.z, rb.z));
+                                return Rotated{fma2(pack2(rb.w, rb.w), pack2(ca.x, ca.y), pack2(rb.x, rb.y)),
+                                               fmaf(rb.w, ca.z, rb.z)};
                             },
                             w, xs);
             } else {
-                acc.add_bearing(a.P, a.src, Acc::val(a.Wf), Acc::val(a.Hf), halfW, halfH, shift, px, py, pz, e.x, e.y,
-                                e.z, w, xs);
+                acc.add_bearing(a.P, a.src, scale, half, shift, px, py, pz, e.x, e.y, e.z, w, xs);
             }
         }
     }
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(kThreads, persistent_min_blocks<S>()) batch_ke
 // from global memory (L1-resident) instead of a staged tile.  Same per-tap
 // arithmetic (TapAccum) as the tile kernel.
 template <int S, class Img>
-__global__ void __launch_bounds__(256) hyp_kernel(const __grid_constant__ HypArgs a) {
+__global__ void __launch_bounds__(256, 2) hyp_kernel(const __grid_constant__ HypArgs a) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= a.n) return;
     const int2 ij = a.ij[h];
@@ -719,7 +719,8 @@ __global__ void __launch_bounds__(256) hyp_kernel(const __grid_constant__ HypArg
     const float Ic = a.ref[(size_t)i * W + j];
     const float px = a.planes[3 * h], py = a.planes[3 * h + 1], pz = a.planes[3 * h + 2];
     const float shift = Img::shift_for(Ic);
-    const float halfW = fmaf(0.5f, a.Wf, Img::kCoordOffset), halfH = fmaf(0.5f, a.Hf, Img::kCoordOffset);
+    const f32x2 scale = pack2(a.Wf, 2.0f * a.Hf);
+    const f32x2 half = pack2(fmaf(0.5f, a.Wf, Img::kCoordOffset), fmaf(0.5f, a.Hf, Img::kCoordOffset));
     float sw = 0.f, swx = 0.f, swxx = 0.f;
     TapAccum<S, Img> acc;
     acc.zero();
@@ -735,7 +736,7 @@ __global__ void __launch_bounds__(256) hyp_kernel(const __grid_constant__ HypArg
             sw += w;
             swx = fmaf(w, xs, swx);
             swxx = fmaf(w * xs, xs, swxx);
-            acc.add_trig(a.P, a.src, a.Wf, a.Hf, halfW, halfH, shift, px, py, pz, rt, ct, w, xs);
+            acc.add_trig(a.P, a.src, scale, half, shift, px, py, pz, rt, ct, w, xs);
         }
     }
     float sep[S], cum[S];

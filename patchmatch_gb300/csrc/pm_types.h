@@ -11,8 +11,10 @@ namespace pm {
 constexpr int kMaxSrc = PM_MAX_SOURCES;
 
 // Composed reference-camera -> source-camera poses, FP64-composed on the
-// host and rounded to float: X_r = M_r X_c + c_r, stored as three rows
-// (M_r[k][0..2], c_r[k]) per source so a row is one 16-byte load.
+// host and rounded to float: X_r = M_r X_c + c_r.  The first two rows are
+// interleaved so that the packed FP32 pairs of the sample loop read both with
+// one aligned 8-byte operand: G[r][0] = (M00, M10, M01, M11),
+// G[r][1] = (M02, M12, c0, c1), G[r][2] = (M20, M21, M22, c2).
 struct PmPoses {
     float4 G[kMaxSrc][3];
 };
