@@ -265,6 +265,7 @@ void pmi::fill_args(pm_request *r) {
     a.cand = r->seed;
     a.score = r->score;
     a.best = r->best;
+    a.changed = reinterpret_cast<uint8_t *>(r->d0);  // post-filter scratch, idle during the sweeps
     a.W = r->W;
     a.H = r->H;
     a.Wf = (float)r->W;
@@ -359,12 +360,13 @@ void set_tile_order(pm_request *r) {
     r->banded_blocks = bps > 0 ? bps * r->ctx->n_sm : 0;
 }
 
-int launch_tile(pm_request *r, int mode, int colour, int sweep, cudaStream_t st = nullptr) {
+int launch_tile(pm_request *r, int mode, int colour, int sweep, cudaStream_t st = nullptr, bool use_changed = false) {
     if (!st) st = r->stream;
     pm::SweepArgs a = r->args;
     a.mode = mode;
     a.colour = colour;
     a.sweep = sweep;
+    a.use_changed = use_changed;
     const int kind = pm::image_kind(r->prm.image_format, r->prm.sampler);
     const dim3 grid = pm::tile_grid(r->W, r->H);
     pm::BandArgs band{};
@@ -401,7 +403,8 @@ int enqueue_init(pm_request *r) {
 
 int enqueue_sweeps(pm_request *r, int first_half, int n_half) {
     for (int h = first_half; h < first_half + n_half; ++h) {
-        int rc = launch_tile(r, pm::kModeSweep, h & 1, h >> 1);
+        // from the third half-sweep on, the two before it have recorded what changed
+        int rc = launch_tile(r, pm::kModeSweep, h & 1, h >> 1, nullptr, h >= first_half + 2);
         if (rc) return rc;
     }
     return PM_OK;

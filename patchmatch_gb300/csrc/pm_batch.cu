@@ -212,6 +212,7 @@ int batch_enqueue(pm_batch *b) {
                 a.mode = ph < 2 ? pm::kModeScore : pm::kModeSweep;
                 a.colour = ph < 2 ? ph : (ph - 2) & 1;
                 a.sweep = ph < 2 ? 0 : (ph - 2) >> 1;
+                a.use_changed = ph >= 4;
                 const dim3 grid = pm::tile_grid(r->W, r->H);
                 pm::BandArgs band{};
                 const pm::BandArgs *bp = nullptr;
@@ -269,6 +270,7 @@ int batch_enqueue(pm_batch *b) {
                 a.mode = mode;
                 a.colour = colour;
                 a.sweep = sweep;
+                a.use_changed = ph >= 4;
                 const bool mixed = b->executor == PM_BATCH_MIXED;
                 const int occ = std::max(1, mixed ? pm::dispatch_batch_mixed_blocks_per_sm(g.kind, g.plain)
                                                   : pm::dispatch_batch_blocks_per_sm(g.S, g.kind, g.plain));
@@ -283,6 +285,7 @@ int batch_enqueue(pm_batch *b) {
                     a.mode = mode;
                     a.colour = colour;
                     a.sweep = sweep;
+                    a.use_changed = ph >= 4;
                     const dim3 grid = pm::tile_grid(a.W, a.H);
                     pm::BandArgs band{};
                     const pm::BandArgs *bp = nullptr;

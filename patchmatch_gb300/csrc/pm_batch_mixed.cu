@@ -23,11 +23,11 @@ using MixedImg = typename std::conditional<
 
 template <int S, bool Plain>
 __device__ __forceinline__ void visit(const SweepArgs &sa, int bx, int by, float4 *tile) {
-    tile_body<S, MixedImg, Plain, SharedAccess>(sa, bx, by, tile);
+    tile_body<S, MixedImg, Plain, kTileH, SharedAccess>(sa, bx, by, tile);
 }
 
 template <bool Plain>
-__global__ void __launch_bounds__(kThreads, 2 * kCtaScale) batch_mixed_kernel(const __grid_constant__ BatchArgs b) {
+__global__ void __launch_bounds__(Geo<kTileH>::kThreads, 2) batch_mixed_kernel(const __grid_constant__ BatchArgs b) {
     extern __shared__ float4 tile[];
     __shared__ SweepArgs sa;
     __shared__ int s_item;
@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(kThreads, 2 * kCtaScale) batch_mixed_kernel(co
             sa.mode = b.mode;
             sa.colour = b.colour;
             sa.sweep = b.sweep;
+            sa.use_changed = b.use_changed;
         }
         __syncthreads();
         switch (w.w) {
@@ -68,9 +69,9 @@ __global__ void __launch_bounds__(kThreads, 2 * kCtaScale) batch_mixed_kernel(co
 template <>
 cudaError_t launch_batch_mixed<PM_MIXED_KIND>(bool plain, int blocks, cudaStream_t st, const BatchArgs &b) {
     if (plain)
-        batch_mixed_kernel<true><<<blocks, kThreads, tile_kernel_smem_max(), st>>>(b);
+        batch_mixed_kernel<true><<<blocks, Geo<kTileH>::kThreads, tile_kernel_smem_max(), st>>>(b);
     else
-        batch_mixed_kernel<false><<<blocks, kThreads, tile_kernel_smem_max(), st>>>(b);
+        batch_mixed_kernel<false><<<blocks, Geo<kTileH>::kThreads, tile_kernel_smem_max(), st>>>(b);
     return cudaGetLastError();
 }
 
@@ -85,9 +86,9 @@ template <>
 int batch_mixed_blocks_per_sm<PM_MIXED_KIND>(bool plain) {
     int n = 0;
     if (plain)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<true>, kThreads, tile_kernel_smem_max());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<true>, Geo<kTileH>::kThreads, tile_kernel_smem_max());
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<false>, kThreads, tile_kernel_smem_max());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<false>, Geo<kTileH>::kThreads, tile_kernel_smem_max());
     return n;
 }
 

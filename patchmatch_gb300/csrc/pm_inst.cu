@@ -10,6 +10,8 @@
 namespace pm {
 
 namespace {
+constexpr int kThreads = Geo<kTileH>::kThreads;
+
 template <class Img>
 cudaError_t tile_launch(dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band) {
     if (band) {

@@ -38,9 +38,11 @@ struct SweepArgs {
     const float4 *cand;         // H x W seeding candidates (w = depth, 0 = none), mode kModeSeed
     float *score;               // H x W
     int8_t *best;               // H x W
+    uint8_t *changed;           // H x W: whether the pixel's last visit changed its state
     int W, H;
     float Wf, Hf;
     int patch_half;
+    int use_changed;            // the two half-sweeps before this one filled `changed` in
     int colour;                 // 0 = red, 1 = black: pixels with (i + j + colour) even
     int sweep;                  // sweep index (Philox tag = sweep + 1)
     int mode;                   // 0 = score own plane, 1 = red-black update
@@ -77,7 +79,7 @@ struct BatchArgs {
     const int4 *items;       // (request, tile x, tile y, 0), request-major
     int n_items;
     unsigned int *counter;   // next item; zero before the launch
-    int mode, colour, sweep;
+    int mode, colour, sweep, use_changed;
 };
 
 // kModeScore: score each pixel's own plane; kModeSweep: red-black update;
