@@ -98,8 +98,6 @@ int __float_as_int_host(float f) {
     return i;
 }
 
-// Start alignment of the per-source sampling buffers: texture objects bound
-// to pitched linear memory need the device's texture alignment (512 bytes).
 constexpr int kMaxBands = 1024;  // counters of the banded tile order (one per SM)
 // The banded tile order (BandArgs) pays when the sources' texture rows are
 // wide: the CTAs resident on an SM then overflow L1 with unrelated tiles'
@@ -115,6 +113,17 @@ constexpr int kMaxBands = 1024;  // counters of the banded tile order (one per S
 constexpr size_t kBandedMinRowBytes = 30000;
 constexpr size_t kBandedMinRowBytesWide = 21000;  // W >= 2880, up to 7 sources
 constexpr int kBandedWideW = 2880;
+// Images of at most this many tile rows (warps) per SM run tile_kernel_small
+// (its 16 warps per SM hold them in about one wave).  Measured against the
+// large-tile kernel, 8 sweeps, time ratio with 2 / 4 / 6 / 8 sources, textures:
+// 448x224 (10 warps per SM) 0.73 / 0.86 / 0.81 / 0.87, 512x256 (13)
+// 0.84 / 0.95 / 0.98 / 1.03, 576x288 (17) 0.93 / 0.95 / 0.92 / 0.97, 640x320
+// (21) 1.00 / 1.06 / 1.07 / 0.97.  The quad samplers, whose loads and bilinear
+// weights take more registers, gain up to 384x192 (8): 2 / 5 / 8 sources
+// 0.75 / 0.94 / 0.99, 512x256 0.95 / 1.03 / 1.02.
+constexpr int kSmallWarpsTexture = 18, kSmallWarpsQuad = 12;
+// Start alignment of the per-source sampling buffers: texture objects bound
+// to pitched linear memory need the device's texture alignment (512 bytes).
 constexpr size_t kTexAlign = 512;
 
 int get_trig(pm_ctx *ctx, int W, int H, Trig *out) {
@@ -345,13 +354,20 @@ int ensure_textures(pm_request *r) {
     return PM_OK;
 }
 
-// Choose the tile order of a request: banded (persistent grid) for texture
+// Choose the tile height and order of a request: small tiles for images that
+// fit the chip at once (kSmallWarps*); else banded (persistent grid) for texture
 // sampling when the sources' row bytes W x bytes per texel x S reach
 // kBandedMinRowBytes (kBandedMinRowBytesWide from kBandedWideW pixels wide
 // with up to 7 sources), else one CTA per tile (the quad samplers measured
 // 4-6 % slower banded at 1920x960).
 void set_tile_order(pm_request *r) {
     r->banded_blocks = 0;
+    // all tiles resident at once: the latency of one tile visit counts
+    const int max_warps = r->prm.sampler == PM_SAMPLER_TEXTURE ? kSmallWarpsTexture : kSmallWarpsQuad;
+    const long long warps = (long long)((r->W + pm::kTileWidth - 1) / pm::kTileWidth) * r->H;
+    r->tile_rows = r->S <= pm::kSmallMaxSources && warps <= (long long)max_warps * r->ctx->n_sm ? pm::kTileRowsSmall
+                                                                                                : pm::kTileRowsLarge;
+    if (r->tile_rows == pm::kTileRowsSmall) return;
     if (r->ctx->n_sm <= 0 || r->ctx->n_sm > kMaxBands / 2 || r->prm.sampler != PM_SAMPLER_TEXTURE) return;
     const size_t texel = r->prm.image_format == PM_IMAGE_F16 ? 2 : 1;
     const size_t min_row = (r->W >= kBandedWideW && r->S <= 7) ? kBandedMinRowBytesWide : kBandedMinRowBytes;
@@ -368,12 +384,12 @@ int launch_tile(pm_request *r, int mode, int colour, int sweep, cudaStream_t st 
     a.sweep = sweep;
     a.use_changed = use_changed;
     const int kind = pm::image_kind(r->prm.image_format, r->prm.sampler);
-    const dim3 grid = pm::tile_grid(r->W, r->H);
+    const dim3 grid = pm::tile_grid(r->W, r->H, r->tile_rows);
     pm::BandArgs band{};
     const pm::BandArgs *bp = nullptr;
     const int rc = pmi::tile_band(r, grid, st, &band, &bp);
     if (rc) return rc;
-    cudaError_t e = pm::dispatch_tile(r->S, kind, grid, st, a, bp);
+    cudaError_t e = pm::dispatch_tile(r->S, kind, r->tile_rows, grid, st, a, bp);
     r->ctx->launches++;
     if (e != cudaSuccess) return fail(r->ctx, PM_ECUDA, "tile kernel launch: %s", cudaGetErrorString(e));
     return PM_OK;
@@ -590,20 +606,23 @@ int enqueue_run(pm_request *r) {
 }  // namespace
 
 namespace pm {
-dim3 tile_grid(int W, int H) { return dim3((W + kTileW - 1) / kTileW, (H + kTileH - 1) / kTileH); }
+const int kTileWidth = kTileW, kTileRowsLarge = kTileH, kTileRowsSmall = kSmallH;
 
-cudaError_t dispatch_tile(int S, int kind, dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band) {
+dim3 tile_grid(int W, int H, int rows) { return dim3((W + kTileW - 1) / kTileW, (H + rows - 1) / rows); }
+
+cudaError_t dispatch_tile(int S, int kind, int rows, dim3 grid, cudaStream_t st, const SweepArgs &a,
+                          const BandArgs *band) {
     switch (S) {
-        case 1: return launch_tile<1>(kind, grid, st, a, band);
-        case 2: return launch_tile<2>(kind, grid, st, a, band);
-        case 3: return launch_tile<3>(kind, grid, st, a, band);
-        case 4: return launch_tile<4>(kind, grid, st, a, band);
-        case 5: return launch_tile<5>(kind, grid, st, a, band);
-        case 6: return launch_tile<6>(kind, grid, st, a, band);
-        case 7: return launch_tile<7>(kind, grid, st, a, band);
-        case 8: return launch_tile<8>(kind, grid, st, a, band);
-        case 9: return launch_tile<9>(kind, grid, st, a, band);
-        case 10: return launch_tile<10>(kind, grid, st, a, band);
+        case 1: return launch_tile<1>(kind, rows, grid, st, a, band);
+        case 2: return launch_tile<2>(kind, rows, grid, st, a, band);
+        case 3: return launch_tile<3>(kind, rows, grid, st, a, band);
+        case 4: return launch_tile<4>(kind, rows, grid, st, a, band);
+        case 5: return launch_tile<5>(kind, rows, grid, st, a, band);
+        case 6: return launch_tile<6>(kind, rows, grid, st, a, band);
+        case 7: return launch_tile<7>(kind, rows, grid, st, a, band);
+        case 8: return launch_tile<8>(kind, rows, grid, st, a, band);
+        case 9: return launch_tile<9>(kind, rows, grid, st, a, band);
+        case 10: return launch_tile<10>(kind, rows, grid, st, a, band);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -128,7 +128,7 @@ int batch_build(pm_batch *b) {
     for (auto &g : b->groups) {
         std::vector<int4> items;
         for (int m = 0; m < (int)g.members.size(); ++m) {
-            const dim3 tg = pm::tile_grid(g.members[m]->W, g.members[m]->H);
+            const dim3 tg = pm::tile_grid(g.members[m]->W, g.members[m]->H, pm::kTileRowsLarge);
             for (unsigned y = 0; y < tg.y; ++y)
                 for (unsigned x = 0; x < tg.x; ++x) items.push_back(make_int4(m, (int)x, (int)y, g.members[m]->S));
         }
@@ -213,12 +213,12 @@ int batch_enqueue(pm_batch *b) {
                 a.colour = ph < 2 ? ph : (ph - 2) & 1;
                 a.sweep = ph < 2 ? 0 : (ph - 2) >> 1;
                 a.use_changed = ph >= 4;
-                const dim3 grid = pm::tile_grid(r->W, r->H);
+                const dim3 grid = pm::tile_grid(r->W, r->H, r->tile_rows);
                 pm::BandArgs band{};
                 const pm::BandArgs *bp = nullptr;
                 const int rc = pmi::tile_band(r, grid, bs, &band, &bp);
                 if (rc) return rc;
-                cudaError_t e = pm::dispatch_tile(r->S, kind, grid, bs, a, bp);
+                cudaError_t e = pm::dispatch_tile(r->S, kind, r->tile_rows, grid, bs, a, bp);
                 if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
                 ++launches;
             }
@@ -286,12 +286,13 @@ int batch_enqueue(pm_batch *b) {
                     a.colour = colour;
                     a.sweep = sweep;
                     a.use_changed = ph >= 4;
-                    const dim3 grid = pm::tile_grid(a.W, a.H);
+                    const int rows = g.members[m]->tile_rows;
+                    const dim3 grid = pm::tile_grid(a.W, a.H, rows);
                     pm::BandArgs band{};
                     const pm::BandArgs *bp = nullptr;
                     const int rc = pmi::tile_band(g.members[m], grid, st, &band, &bp);
                     if (rc) return rc;
-                    cudaError_t e = pm::dispatch_tile(g.S, g.kind, grid, st, a, bp);
+                    cudaError_t e = pm::dispatch_tile(g.S, g.kind, rows, grid, st, a, bp);
                     if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
                     ++launches;
                 }

@@ -23,7 +23,7 @@ using MixedImg = typename std::conditional<
 
 template <int S, bool Plain>
 __device__ __forceinline__ void visit(const SweepArgs &sa, int bx, int by, float4 *tile) {
-    tile_body<S, MixedImg, Plain, kTileH, SharedAccess>(sa, bx, by, tile);
+    tile_body<S, MixedImg, Plain, kTileH, 1, SharedAccess>(sa, bx, by, tile);
 }
 
 template <bool Plain>

@@ -13,7 +13,18 @@ namespace {
 constexpr int kThreads = Geo<kTileH>::kThreads;
 
 template <class Img>
-cudaError_t tile_launch(dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band) {
+cudaError_t tile_launch(int rows, dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band) {
+    if (rows == kSmallH) {
+        if constexpr (PM_INST_S <= kSmallMaxSources) {
+            constexpr size_t smem = tile_kernel_smem<PM_INST_S, kSmallH>();
+            if (a.propagation == PM_PROPAGATION_PLAIN)
+                tile_kernel_small<PM_INST_S, Img, true><<<grid, Geo<kSmallH>::kThreads, smem, st>>>(a);
+            else
+                tile_kernel_small<PM_INST_S, Img, false><<<grid, Geo<kSmallH>::kThreads, smem, st>>>(a);
+            return cudaGetLastError();
+        }
+        return cudaErrorInvalidValue;
+    }
     if (band) {
         if (a.propagation == PM_PROPAGATION_PLAIN)
             tile_kernel_banded<PM_INST_S, Img, true><<<band->blocks, kThreads, tile_kernel_smem<PM_INST_S>(), st>>>(
@@ -28,6 +39,13 @@ cudaError_t tile_launch(dim3 grid, cudaStream_t st, const SweepArgs &a, const Ba
     else
         tile_kernel<PM_INST_S, Img, false><<<grid, kThreads, tile_kernel_smem<PM_INST_S>(), st>>>(a);
     return cudaGetLastError();
+}
+
+template <class K>
+cudaError_t small_attr(K kernel) {
+    constexpr int dyn = (int)tile_kernel_smem<PM_INST_S, kSmallH>();
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+    return e ? e : prefer_l1(kernel, dyn, kSmallMinBlocks);
 }
 
 template <class Img>
@@ -47,6 +65,10 @@ cudaError_t tile_smem_attr() {
     e = e ? e : cudaFuncSetAttribute(tile_kernel_banded<PM_INST_S, Img, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
     e = e ? e : prefer_l1(tile_kernel_banded<PM_INST_S, Img, false>, dyn, pblocks);
+    if constexpr (PM_INST_S <= kSmallMaxSources) {
+        e = e ? e : small_attr(tile_kernel_small<PM_INST_S, Img, false>);
+        e = e ? e : small_attr(tile_kernel_small<PM_INST_S, Img, true>);
+    }
     return e ? e : prefer_l1(tile_kernel_banded<PM_INST_S, Img, true>, dyn, pblocks);
 }
 
@@ -99,12 +121,13 @@ cudaError_t configure_tile<PM_INST_S>() {
 
 // kind: kImageQuadU8, kImageQuadF16, kImageTexU8, kImageTexF16
 template <>
-cudaError_t launch_tile<PM_INST_S>(int kind, dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band) {
+cudaError_t launch_tile<PM_INST_S>(int kind, int rows, dim3 grid, cudaStream_t st, const SweepArgs &a,
+                                   const BandArgs *band) {
     switch (kind) {
-        case kImageQuadF16: return tile_launch<QuadF16>(grid, st, a, band);
-        case kImageTexU8: return tile_launch<TexU8>(grid, st, a, band);
-        case kImageTexF16: return tile_launch<TexF16>(grid, st, a, band);
-        default: return tile_launch<QuadU8>(grid, st, a, band);
+        case kImageQuadF16: return tile_launch<QuadF16>(rows, grid, st, a, band);
+        case kImageTexU8: return tile_launch<TexU8>(rows, grid, st, a, band);
+        case kImageTexF16: return tile_launch<TexF16>(rows, grid, st, a, band);
+        default: return tile_launch<QuadU8>(rows, grid, st, a, band);
     }
 }
 

@@ -59,6 +59,7 @@ struct pm_request {
     int W = 0, H = 0, S = 0;
     int batch_refs = 0;  // batches holding this request (it cannot be destroyed meanwhile)
     unsigned *band_ctr = nullptr;  // per-SM tile counters of the banded order (in the block)
+    int tile_rows = 8;             // tile height of its launches
     int banded_blocks = 0;         // persistent grid of the banded order (0: one CTA per tile)
     pm_params prm{};
     size_t bytes = 0;

@@ -27,7 +27,7 @@ inline int image_kind(int image_format, int sampler) {
 // pm_inst.cu (one translation unit per source count S)
 // band: null for one CTA per tile over `grid`, else the banded persistent order
 template <int S>
-cudaError_t launch_tile(int kind, dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band);
+cudaError_t launch_tile(int kind, int rows, dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band);
 template <int S>
 int tile_blocks_per_sm(int kind);
 template <int S>
@@ -45,12 +45,15 @@ template <int Kind>
 cudaError_t configure_batch_mixed();  // dynamic shared-memory limit of the current device
 cudaError_t dispatch_batch_mixed(int kind, bool plain, int blocks, cudaStream_t st, const BatchArgs &b);
 int dispatch_batch_mixed_blocks_per_sm(int kind, bool plain);
-cudaError_t dispatch_tile(int S, int kind, dim3 grid, cudaStream_t st, const SweepArgs &a, const BandArgs *band);
+// rows: tile height of the grid (kTileH or kSmallH of pm_sweep.cuh)
+cudaError_t dispatch_tile(int S, int kind, int rows, dim3 grid, cudaStream_t st, const SweepArgs &a,
+                          const BandArgs *band);
 int dispatch_tile_blocks_per_sm(int S, int kind);
 cudaError_t dispatch_batch(int S, int kind, bool plain, int blocks, cudaStream_t st, const BatchArgs &b);
 int dispatch_batch_blocks_per_sm(int S, int kind, bool plain);
 cudaError_t dispatch_hyp(int S, int kind, int n, cudaStream_t st, const HypArgs &a);
-dim3 tile_grid(int W, int H);
+dim3 tile_grid(int W, int H, int rows);  // one CTA per 64-column tile of `rows` rows
+extern const int kTileWidth, kTileRowsLarge, kTileRowsSmall;  // tile width and the two tile heights
 
 // pm_seed.cu: prior result -> seeding candidates of a new keyframe
 struct WarpArgs {

@@ -19,7 +19,8 @@
 
 namespace pm {
 constexpr int kTileW = 64;
-constexpr int kTileH = 8;   // rows per tile = warps per CTA
+constexpr int kTileH = 8;   // rows per tile = warps per CTA of the other kernels
+constexpr int kSmallH = 4;  // the same of the small-image kernel (tile_kernel_small)
 constexpr int kHaloMax = 5;                             // largest supported patch_half
 constexpr int kTileCols = (kTileW + 2 * kHaloMax) / 2;  // 37 same-colour entries per row
 constexpr int kMaxTaps = (kHaloMax + 1) * (kHaloMax + 1);
@@ -189,15 +190,15 @@ struct Park {
 // texture samples (measured, 8 sweeps, 8 sources: 3840x1920 FP16 banded
 // 444 -> 384 ms, u8 at 960x480 to 3840x1920 1-3 % faster; 7 sources at
 // 1920x960 u8 1 % slower with 2).  The one-CTA-per-tile kernel runs 4 (64
-// registers, no spills) up to 4 sources, where the extra warps hide more
-// texture latency (measured, 8 sweeps at 1920x960: 2 sources 3 %, 3 sources
-// 1 %, 4 sources 3 % faster; 5-6 sources spill and run 1-3 % slower).  The
-// persistent kernels (banded, batched) keep 3 there: at 64 registers they
-// spill.
+// registers) for 1 and 2 sources, where the extra warps hide more texture
+// latency (1920x960, 8 sweeps: 17.1 -> 15.9 and 23.4 -> 22.6 ms); with 3 and
+// 4 sources it would spill there and 3 CTAs are as fast or faster (512x256:
+// 3.96 -> 3.70 and 4.88 -> 4.58 ms, 1920x960 and 2880x1440 within 0.5 %).
+// The persistent kernels (banded, batched) keep 3 there.
 template <int S>
 constexpr int persistent_min_blocks() { return S <= 7 ? 3 : 2; }
 template <int S>
-constexpr int tile_min_blocks() { return S <= 4 ? 4 : persistent_min_blocks<S>(); }
+constexpr int tile_min_blocks() { return S <= 2 ? 4 : persistent_min_blocks<S>(); }
 
 // Smoothness factor f in [0, 1] of a propagated plane p against the pixel's
 // current plane h and its depth before propagation (PatchMatchCuda.cu:322-337).
@@ -253,9 +254,9 @@ __device__ __forceinline__ bool nbr_inside(int n, int i, int j, int W, int H) {
 }
 
 // Window moments of plane (px, py, pz) at a pixel: the 36 taps x S sources of
-// the plane-induced warp (PatchMatchCuda.cu:100-157), one tap row and column
-// at a time from the staged tile.
-template <int S, class Img, int TH, class Acc, class A>
+// the plane-induced warp (PatchMatchCuda.cu:100-157), one tap row and U
+// columns at a time from the staged tile.
+template <int S, class Img, int TH, int U, class Acc, class A>
 __device__ __forceinline__ void accumulate_plane(TapAccum<S, Img, Acc> &acc, const A &a, const float4 *tile,
                                                  const float4 *fac, int rbase, int cbase, int pa, float Ic, float px,
                                                  float py, float pz) {
@@ -271,7 +272,7 @@ __device__ __forceinline__ void accumulate_plane(TapAccum<S, Img, Acc> &acc, con
         const float4 *trow = tile + tr * kTileCols + cbase;
         const int k1 = 2 * m1 - ph;
         const float dk1 = (float)(k1 * k1) * Acc::val(a.ndf);
-#pragma unroll 1
+#pragma unroll U
         for (int m2 = 0; m2 < nt; ++m2) {
             const float4 e = trow[m2];
             const int k2 = 2 * m2 - ph;
@@ -332,7 +333,7 @@ constexpr unsigned kScored = 8;
 // combination before the smoothness factor) and best sources land in
 // res/res_best[n][pixel], and flag[pixel] gets the outcome against the
 // pixel's parked score.  All threads of the CTA call it together.
-template <int S, class Img, int TH, class Acc, class A>
+template <int S, class Img, int TH, int U, class Acc, class A>
 __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const float4 *fac, unsigned char *smem,
                                            int i0, int x0, unsigned need) {
     using G = Geo<TH>;
@@ -355,7 +356,7 @@ __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const
             const TilePixel g(p, i0, x0, a.colour, a.patch_half);
             const float4 np = a.plane[nbr_index(n, g.i, g.j, a.W)];
             TapAccum<S, Img, Acc> acc;
-            accumulate_plane<S, Img, TH, Acc>(acc, a, tile, fac, g.rbase, g.cbase, g.pa, tile[g.ctr_e].w, np.x, np.y,
+            accumulate_plane<S, Img, TH, U, Acc>(acc, a, tile, fac, g.rbase, g.cbase, g.pa, tile[g.ctr_e].w, np.x, np.y,
                                                  np.z);
             e = list[q];
             p = e >> 3;
@@ -403,7 +404,7 @@ __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const
 // half of them from the fourth sweep on (0.6 of 1.2 per pixel in the last).
 // Measured, 8 sweeps, both together: 1920x960, 6 sources 58.0 -> 53.4 ms;
 // 512x256, 4 sources 5.06 -> 4.4 ms.
-template <int S, class Img, bool Plain, int TH, class Acc, class A>
+template <int S, class Img, bool Plain, int TH, int U, class Acc, class A>
 __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *tile) {
     using G = Geo<TH>;
     constexpr int kThreads = G::kThreads;
@@ -510,7 +511,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
 #pragma unroll 1
         while (__syncthreads_or(need != 0)) {
             park.save(hx, hy, hz, score, best | (n << 8), curr_depth);
-            spec_round<S, Img, TH, Acc>(a, tile, fac, smem, i0, x0, need);
+            spec_round<S, Img, TH, U, Acc>(a, tile, fac, smem, i0, x0, need);
             unsigned known;
             {
                 int st;
@@ -651,7 +652,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
 
         // ---- cost of hypothesis (px, py, pz) ----
         TapAccum<S, Img, Acc> acc;
-        accumulate_plane<S, Img, TH, Acc>(acc, a, tile, fac, rbase, cbase, pa, Ic, px, py, pz);
+        accumulate_plane<S, Img, TH, U, Acc>(acc, a, tile, fac, rbase, cbase, pa, Ic, px, py, pz);
         {
             int st, ij;
             park.load(hx, hy, hz, cx, cy, cz, score, current_depth, depth_hyp, f, sw, swx, swxx, curr_depth, cand_w, st,
@@ -716,7 +717,28 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
 template <int S, class Img, bool Plain>
 __global__ void __launch_bounds__(Geo<kTileH>::kThreads, tile_min_blocks<S>()) tile_kernel(const __grid_constant__ SweepArgs a) {
     extern __shared__ float4 tile[];
-    tile_body<S, Img, Plain, kTileH, ParamAccess>(a, blockIdx.x, blockIdx.y, tile);
+    tile_body<S, Img, Plain, kTileH, 1, ParamAccess>(a, blockIdx.x, blockIdx.y, tile);
+}
+
+// The same visit for images whose tiles all fit the chip at once (the rule is
+// in pm_api.cu, set_tile_order).  There a half-sweep lasts as long as one
+// tile's chain of costs, so the tiles have 4 rows (twice as many SMs get one),
+// and a lane runs two taps' worth of chains side by side, in the 128 registers
+// that 16 warps per SM leave each thread (from 7 sources one tap fills them).
+// Measured, 8 sweeps, against the kernel above: 256x128 2 sources 2.08 ->
+// 1.43 ms, 4 sources 3.34 -> 2.10 ms; 448x224 4 sources 4.07 -> 3.49 ms;
+// 512x256 2 sources 3.05 -> 2.55 ms, 4 sources 4.48 -> 4.27 ms.  Tiles of 2
+// rows (4.65 ms at 512x256 with 4 sources) and 1 row (4.81 ms) lose more to
+// their halos and part-filled lists; three taps at once spill from 5 sources.
+template <int S>
+__host__ __device__ constexpr int small_taps() { return S <= 6 ? 2 : 1; }
+constexpr int kSmallMinBlocks = 4;
+constexpr int kSmallMaxSources = 8;  // with 9 and 10 (factored warp) 333x167 is even or 7 % slower in small tiles
+template <int S, class Img, bool Plain>
+__global__ void __launch_bounds__(Geo<kSmallH>::kThreads, kSmallMinBlocks)
+    tile_kernel_small(const __grid_constant__ SweepArgs a) {
+    extern __shared__ float4 tile[];
+    tile_body<S, Img, Plain, kSmallH, small_taps<S>(), ParamAccess>(a, blockIdx.x, blockIdx.y, tile);
 }
 
 // Banded tile order (BandArgs): the same tile visit in a persistent grid.
@@ -750,7 +772,7 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S
         const int t = s_tile;
         if (t < 0) return;
         const int ty = t / b.tiles_x;
-        tile_body<S, Img, Plain, kTileH, ParamAccess>(a, t - ty * b.tiles_x, ty, tile);
+        tile_body<S, Img, Plain, kTileH, 1, ParamAccess>(a, t - ty * b.tiles_x, ty, tile);
         __syncthreads();  // before the next tile replaces the staged tile and s_tile
     }
 }
@@ -784,7 +806,7 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S
             sa.use_changed = b.use_changed;
         }
         __syncthreads();
-        tile_body<S, Img, Plain, kTileH, SharedAccess>(sa, w.y, w.z, tile);
+        tile_body<S, Img, Plain, kTileH, 1, SharedAccess>(sa, w.y, w.z, tile);
         __syncthreads();  // before the next item replaces the arguments and the tile
     }
 }
