@@ -208,100 +208,181 @@ __global__ void clean_kernel(const __grid_constant__ CleanArgs a) {
 // original value.  Processing views in order with an atomicMin per target
 // reproduces that exactly, independent of thread scheduling.
 // ---------------------------------------------------------------------------
+//
+// All of these kernels move a few bytes per pixel; with one pixel per thread
+// they waited for their own dependent loads.  A thread takes V = 4 consecutive
+// pixels with vector accesses and keeps their gathers in flight together;
+// V = 1 where rows or maps are not aligned for that.  Measured at 3840x1920
+// with 5 views (one pixel -> four per thread, us): init 33 -> 15, classify
+// 59/51/43/40 -> 48/42/35/31 (bound by the projection's arithmetic), resolve
+// 47/41/35/33 -> 23/17/15/14, count 21 -> 4, scan 14 -> 5, scatter 38 -> 15.
 enum : int8_t { kSkip = 0, kZero = 1, kDrop = 2 };
 
-__global__ void fuse_init_kernel(const __grid_constant__ FuseArgs a) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= a.H || j >= a.W) return;
-    const size_t idx = (size_t)i * a.W + j;
-    const float *D0 = a.depths[0];
-    const float d = D0[idx];
-    bool f = d == 0.0f;
-    if (i - 1 > 0 && i - 1 < a.H) f = f || D0[idx - a.W] == 0.0f;
-    if (j - 1 > 0 && j - 1 < a.W) f = f || D0[idx - 1] == 0.0f;
-    if (i + 1 > 0 && i + 1 < a.H) f = f || D0[idx + a.W] == 0.0f;
-    if (j + 1 > 0 && j + 1 < a.W) f = f || D0[idx + 1] == 0.0f;
-    a.alive[idx] = f ? 0 : 1;
-    a.pruned[idx] = f ? 0.0f : d;
+template <int V, class T>
+struct alignas(sizeof(T) * V) Vec {
+    T v[V];
+};
+template <int V, class T>
+__device__ __forceinline__ Vec<V, T> load_vec(const T *p) {
+    return *reinterpret_cast<const Vec<V, T> *>(p);
+}
+template <int V, class T>
+__device__ __forceinline__ void store_vec(T *p, const Vec<V, T> &x) {
+    *reinterpret_cast<Vec<V, T> *>(p) = x;
 }
 
+template <int V>
+__global__ void fuse_init_kernel(const __grid_constant__ FuseArgs a) {
+    const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * V, i = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= a.H || j0 >= a.W) return;
+    const size_t idx = (size_t)i * a.W + j0;
+    const float *D0 = a.depths[0];
+    const Vec<V, float> d = load_vec<V>(D0 + idx);
+    Vec<V, float> up, down;
+    const bool has_up = i - 1 > 0, has_down = i + 1 < a.H;
+    if (has_up) up = load_vec<V>(D0 + idx - a.W);
+    if (has_down) down = load_vec<V>(D0 + idx + a.W);
+    const float left = j0 - 1 > 0 ? D0[idx - 1] : 1.0f, right = j0 + V < a.W ? D0[idx + V] : 1.0f;
+    Vec<V, uint8_t> alive;
+    Vec<V, float> pruned;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        const int j = j0 + k;
+        bool f = d.v[k] == 0.0f;
+        if (has_up) f = f || up.v[k] == 0.0f;
+        if (has_down) f = f || down.v[k] == 0.0f;
+        if (j - 1 > 0) f = f || (k ? d.v[k ? k - 1 : 0] : left) == 0.0f;
+        if (j + 1 < a.W) f = f || (k + 1 < V ? d.v[k + 1 < V ? k + 1 : 0] : right) == 0.0f;
+        alive.v[k] = f ? 0 : 1;
+        pruned.v[k] = f ? 0.0f : d.v[k];
+    }
+    store_vec(a.alive + idx, alive);
+    store_vec(a.pruned + idx, pruned);
+}
+
+template <int V>
 __global__ void fuse_classify_kernel(const __grid_constant__ FuseArgs a, int k) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= a.H || j >= a.W) return;
-    const size_t idx = (size_t)i * a.W + j;
-    int8_t cls = kSkip;
-    if (a.alive[idx]) {
-        const float d = a.depths[0][idx];
-        const float2 rt = a.row_trig[i], ct = a.col_trig[j];
-        const float Xc = d * rt.x * ct.x, Yc = -d * rt.y, Zc = d * rt.x * ct.y;
-        const float *M = a.M[k], *c = a.c[k];
-        const float X = M[0] * Xc + M[1] * Yc + M[2] * Zc + c[0];
-        const float Y = M[3] * Xc + M[4] * Yc + M[5] * Zc + c[1];
-        const float Z = M[6] * Xc + M[7] * Yc + M[8] * Zc + c[2];
-        float x, y, dop;
-        if (project(X, Y, Z, (float)a.W, (float)a.H, x, y, dop)) {
-            const int iu = (int)x, iv = (int)y;
-            if (iv >= 0 && iv < a.H && iu >= 0 && iu < a.W && !(dop < 1e-5f)) {
-                const int q = iv * a.W + iu;
-                const float dat = a.depths[k][q];
-                if (!(dat == 0.0f || fabsf(dat - dop) > a.thr * dop)) {
-                    cls = d < dat ? kZero : kDrop;
-                    a.target[idx] = q;
-                    if (cls == kZero) atomicMin(a.first + q, (unsigned)idx);
-                }
+    const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * V, i = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= a.H || j0 >= a.W) return;
+    const size_t idx = (size_t)i * a.W + j0;
+    const Vec<V, uint8_t> alive = load_vec<V>(a.alive + idx);
+    const Vec<V, float> d = load_vec<V>(a.depths[0] + idx);
+    const float2 rt = a.row_trig[i];
+    const float *M = a.M[k], *c = a.c[k];
+    Vec<V, int> q;
+    Vec<V, int8_t> cls;
+    float dop[V], dat[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        q.v[v] = -1;
+        if (alive.v[v]) {
+            const float2 ct = a.col_trig[j0 + v];
+            const float Xc = d.v[v] * rt.x * ct.x, Yc = -d.v[v] * rt.y, Zc = d.v[v] * rt.x * ct.y;
+            const float X = M[0] * Xc + M[1] * Yc + M[2] * Zc + c[0];
+            const float Y = M[3] * Xc + M[4] * Yc + M[5] * Zc + c[1];
+            const float Z = M[6] * Xc + M[7] * Yc + M[8] * Zc + c[2];
+            float x, y;
+            if (project(X, Y, Z, (float)a.W, (float)a.H, x, y, dop[v])) {
+                const int iu = (int)x, iv = (int)y;
+                if (iv >= 0 && iv < a.H && iu >= 0 && iu < a.W && !(dop[v] < 1e-5f)) q.v[v] = iv * a.W + iu;
             }
         }
     }
-    a.cls[idx] = cls;
-}
-
-__global__ void fuse_resolve_kernel(const __grid_constant__ FuseArgs a, int k) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= a.H || j >= a.W) return;
-    const size_t idx = (size_t)i * a.W + j;
-    const int8_t cls = a.cls[idx];
-    if (cls == kSkip) return;
-    const int q = a.target[idx];
-    const unsigned f = a.first[q];
-    if ((unsigned)idx > f) return;          // target already zeroed: skipped
-    if ((unsigned)idx == f) {               // first qualifying nearer pixel zeroes it
-        a.depths[k][q] = 0.0f;
-        return;
-    }
-    if (cls == kDrop) {                     // sees the original, farther-or-equal: dropped
-        a.alive[idx] = 0;
-        a.pruned[idx] = 0.0f;
-    }
-}
-
-__global__ void compact_count_kernel(const uint8_t *alive, size_t N, unsigned *counts) {
-    const size_t i = (size_t)blockIdx.x * kCompactBlock + threadIdx.x;
-    const int keep = (i < N) ? alive[i] : 0;
-    const int c = __syncthreads_count(keep);
-    if (threadIdx.x == 0) counts[blockIdx.x] = (unsigned)c;
-}
-
-// exclusive scan of nb block counts (single block); counts[nb] = total
-__global__ void compact_scan_kernel(unsigned *counts, int nb, unsigned *total) {
-    __shared__ unsigned s[1024];
-    __shared__ unsigned carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nb; base += 1024) {
-        const int i = base + threadIdx.x;
-        const unsigned v = i < nb ? counts[i] : 0u;
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            const unsigned t = threadIdx.x >= off ? s[threadIdx.x - off] : 0u;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
+#pragma unroll
+    for (int v = 0; v < V; ++v) dat[v] = q.v[v] >= 0 ? a.depths[k][q.v[v]] : 0.0f;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        cls.v[v] = kSkip;
+        if (q.v[v] >= 0 && !(dat[v] == 0.0f || fabsf(dat[v] - dop[v]) > a.thr * dop[v])) {
+            cls.v[v] = d.v[v] < dat[v] ? kZero : kDrop;
+            if (cls.v[v] == kZero) atomicMin(a.first + q.v[v], (unsigned)(idx + v));
         }
-        if (i < nb) counts[i] = carry + s[threadIdx.x] - v;
+    }
+    store_vec(a.cls + idx, cls);
+    store_vec(a.target + idx, q);
+}
+
+template <int V>
+__global__ void fuse_resolve_kernel(const __grid_constant__ FuseArgs a, int k) {
+    const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * V, i = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= a.H || j0 >= a.W) return;
+    const size_t idx = (size_t)i * a.W + j0;
+    const Vec<V, int8_t> cls = load_vec<V>(a.cls + idx);
+    const Vec<V, int> q = load_vec<V>(a.target + idx);
+    unsigned first[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) first[v] = cls.v[v] != kSkip ? a.first[q.v[v]] : 0u;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const unsigned me = (unsigned)(idx + v);
+        if (cls.v[v] == kSkip || me > first[v]) continue;  // target already zeroed: skipped
+        if (me == first[v]) {                              // first qualifying nearer pixel zeroes it
+            a.depths[k][q.v[v]] = 0.0f;
+        } else if (cls.v[v] == kDrop) {                    // sees the original, farther-or-equal: dropped
+            a.alive[me] = 0;
+            a.pruned[me] = 0.0f;
+        }
+    }
+}
+
+// Kept pixels of compaction block b (kCompactBlock consecutive pixels): 64
+// threads with 16 flags each, four blocks per CTA.
+__global__ void __launch_bounds__(256) compact_count_kernel(const uint8_t *alive, size_t N, unsigned *counts) {
+    __shared__ unsigned part[8];
+    const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 16;
+    unsigned c = 0;
+    if (i + 16 <= N) {
+        const uint4 w = *reinterpret_cast<const uint4 *>(alive + i);  // flags are 0 or 1
+        c = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+    } else {
+        for (size_t k = i; k < N; ++k) c += alive[k];
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
+    __syncthreads();
+    const unsigned b = blockIdx.x * 4 + threadIdx.x;
+    if (threadIdx.x < 4 && (size_t)b * kCompactBlock < N) counts[b] = part[2 * threadIdx.x] + part[2 * threadIdx.x + 1];
+}
+static_assert(kCompactBlock == 1024, "compact_count_kernel sums 64 x 16 flags per block");
+
+// Inclusive prefix sum over a warp.
+__device__ __forceinline__ unsigned warp_scan(unsigned v) {
+    const unsigned lane = threadIdx.x & 31;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, v, off);
+        if (lane >= (unsigned)off) v += t;
+    }
+    return v;
+}
+
+// exclusive scan of nb block counts (single block of 1024, four counts per
+// thread and step); counts[nb] = total
+__global__ void __launch_bounds__(1024) compact_scan_kernel(unsigned *counts, int nb, unsigned *total) {
+    __shared__ unsigned warp_tot[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned carry = 0;
+    for (int base = 0; base < nb; base += 4096) {
+        const int i = base + 4 * (int)threadIdx.x;
+        unsigned v[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = i + k < nb ? counts[i + k] : 0u;
+            sum += v[k];
+        }
+        const unsigned inc = warp_scan(sum);
+        if (lane == 31) warp_tot[wid] = inc;
         __syncthreads();
-        if (threadIdx.x == 1023) carry += s[1023];
-        __syncthreads();
+        const unsigned all = warp_scan(warp_tot[lane]);  // every warp scans the warp totals
+        const unsigned before = wid ? __shfl_sync(0xffffffffu, all, wid - 1) : 0u;
+        unsigned run = carry + before + inc - sum;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i + k < nb) counts[i + k] = run;
+            run += v[k];
+        }
+        carry += __shfl_sync(0xffffffffu, all, 31);
+        __syncthreads();  // before the next step replaces warp_tot
     }
     if (threadIdx.x == 0) {
         counts[nb] = carry;
@@ -309,41 +390,52 @@ __global__ void compact_scan_kernel(unsigned *counts, int nb, unsigned *total) {
     }
 }
 
-__global__ void compact_scatter_kernel(const __grid_constant__ FuseArgs a) {
-    __shared__ unsigned warp_tot[32];
+// Points of compaction block blockIdx.x: 256 threads with 4 pixels each.
+__global__ void __launch_bounds__(256) compact_scatter_kernel(const __grid_constant__ FuseArgs a) {
+    __shared__ unsigned warp_tot[8];
     const size_t N = (size_t)a.W * a.H;
-    const size_t i = (size_t)blockIdx.x * kCompactBlock + threadIdx.x;
-    const int keep = (i < N) ? a.alive[i] : 0;
+    const size_t i0 = (size_t)blockIdx.x * kCompactBlock + 4 * threadIdx.x;
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-    if (lane == 0) warp_tot[wid] = __popc(bal);
+    Vec<4, uint8_t> keep = {};
+    if (i0 + 4 <= N) {
+        keep = load_vec<4>(a.alive + i0);
+    } else {
+        for (int k = 0; k < 4; ++k)
+            if (i0 + k < N) keep.v[k] = a.alive[i0 + k];
+    }
+    const unsigned cnt = keep.v[0] + keep.v[1] + keep.v[2] + keep.v[3];
+    const unsigned inc = warp_scan(cnt);
+    if (lane == 31) warp_tot[wid] = inc;
     __syncthreads();
-    if (wid == 0) {
-        unsigned v = warp_tot[lane];
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned t = __shfl_up_sync(0xffffffffu, v, off);
-            if (lane >= (unsigned)off) v += t;
+    if (!cnt) return;
+    unsigned pos = a.block_counts[blockIdx.x] + inc - cnt;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) pos += w < (int)wid ? warp_tot[w] : 0u;
+    int row = (int)(i0 / a.W), col = (int)(i0 - (size_t)row * a.W);
+    for (int k = 0; k < 4; ++k) {
+        if (keep.v[k]) {
+            const size_t i = i0 + k;
+            const float d = a.depths[0][i];
+            const float2 rt = a.row_trig[row], ct = a.col_trig[col];
+            const float Xc = d * rt.x * ct.x, Yc = -d * rt.y, Zc = d * rt.x * ct.y;
+            a.xyz[3 * (size_t)pos] = a.Rinv[0] * Xc + a.Rinv[1] * Yc + a.Rinv[2] * Zc + a.tw[0];
+            a.xyz[3 * (size_t)pos + 1] = a.Rinv[3] * Xc + a.Rinv[4] * Yc + a.Rinv[5] * Zc + a.tw[1];
+            a.xyz[3 * (size_t)pos + 2] = a.Rinv[6] * Xc + a.Rinv[7] * Yc + a.Rinv[8] * Zc + a.tw[2];
+            if (a.bgr_out && a.bgr) {
+                a.bgr_out[3 * (size_t)pos] = a.bgr[3 * i];
+                a.bgr_out[3 * (size_t)pos + 1] = a.bgr[3 * i + 1];
+                a.bgr_out[3 * (size_t)pos + 2] = a.bgr[3 * i + 2];
+            }
+            if (a.ij_out) {
+                a.ij_out[2 * (size_t)pos] = row;
+                a.ij_out[2 * (size_t)pos + 1] = col;
+            }
+            ++pos;
         }
-        warp_tot[lane] = v - warp_tot[lane];  // exclusive
-    }
-    __syncthreads();
-    if (!keep) return;
-    const unsigned pos = a.block_counts[blockIdx.x] + warp_tot[wid] + __popc(bal & ((1u << lane) - 1u));
-    const int row = (int)(i / a.W), col = (int)(i - (size_t)row * a.W);
-    const float d = a.depths[0][i];
-    const float2 rt = a.row_trig[row], ct = a.col_trig[col];
-    const float Xc = d * rt.x * ct.x, Yc = -d * rt.y, Zc = d * rt.x * ct.y;
-    a.xyz[3 * (size_t)pos] = a.Rinv[0] * Xc + a.Rinv[1] * Yc + a.Rinv[2] * Zc + a.tw[0];
-    a.xyz[3 * (size_t)pos + 1] = a.Rinv[3] * Xc + a.Rinv[4] * Yc + a.Rinv[5] * Zc + a.tw[1];
-    a.xyz[3 * (size_t)pos + 2] = a.Rinv[6] * Xc + a.Rinv[7] * Yc + a.Rinv[8] * Zc + a.tw[2];
-    if (a.bgr_out && a.bgr) {
-        a.bgr_out[3 * (size_t)pos] = a.bgr[3 * i];
-        a.bgr_out[3 * (size_t)pos + 1] = a.bgr[3 * i + 1];
-        a.bgr_out[3 * (size_t)pos + 2] = a.bgr[3 * i + 2];
-    }
-    if (a.ij_out) {
-        a.ij_out[2 * (size_t)pos] = row;
-        a.ij_out[2 * (size_t)pos + 1] = col;
+        if (++col == a.W) {
+            col = 0;
+            ++row;
+        }
     }
 }
 
@@ -413,20 +505,37 @@ void fuse_set_poses(FuseArgs &a, int n, const double *R, const double *t) {
     a.n = n;
 }
 
-cudaError_t launch_fuse(cudaStream_t st, const FuseArgs &a) {
-    dim3 b(32, 8), g((a.W + 31) / 32, (a.H + 7) / 8);
+namespace {
+// Four pixels per thread where every row of every map starts on a 16-byte boundary.
+bool fuse_vector(const FuseArgs &a) {
+    if (a.W % 4) return false;
+    uintptr_t p = (uintptr_t)a.pruned | (uintptr_t)a.target | (uintptr_t)a.depths[0];
+    return (p & 15) == 0 && (((uintptr_t)a.alive | (uintptr_t)a.cls) & 3) == 0;
+}
+
+template <int V>
+cudaError_t launch_fuse_views(cudaStream_t st, const FuseArgs &a) {
+    const dim3 b(32, 8), g((a.W + 32 * V - 1) / (32 * V), (a.H + 7) / 8);
     const size_t N = (size_t)a.W * a.H;
-    fuse_init_kernel<<<g, b, 0, st>>>(a);
+    fuse_init_kernel<V><<<g, b, 0, st>>>(a);
     for (int k = 1; k < a.n; ++k) {
         const cudaError_t e = cudaMemsetAsync(a.first, 0xFF, N * sizeof(unsigned), st);
         if (e != cudaSuccess) return e;
-        fuse_classify_kernel<<<g, b, 0, st>>>(a, k);
-        fuse_resolve_kernel<<<g, b, 0, st>>>(a, k);
+        fuse_classify_kernel<V><<<g, b, 0, st>>>(a, k);
+        fuse_resolve_kernel<V><<<g, b, 0, st>>>(a, k);
     }
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t launch_fuse(cudaStream_t st, const FuseArgs &a) {
+    const size_t N = (size_t)a.W * a.H;
+    const cudaError_t e = fuse_vector(a) ? launch_fuse_views<4>(st, a) : launch_fuse_views<1>(st, a);
+    if (e != cudaSuccess) return e;
     const int nb = compact_blocks(a.W, a.H);
-    compact_count_kernel<<<nb, kCompactBlock, 0, st>>>(a.alive, N, a.block_counts);
+    compact_count_kernel<<<(nb + 3) / 4, 256, 0, st>>>(a.alive, N, a.block_counts);
     compact_scan_kernel<<<1, 1024, 0, st>>>(a.block_counts, nb, a.count);
-    compact_scatter_kernel<<<nb, kCompactBlock, 0, st>>>(a);
+    compact_scatter_kernel<<<nb, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 
