@@ -13,10 +13,12 @@ namespace {
 
 // All of these move a few bytes per pixel and are bound by HBM, once the
 // accesses are wide: a thread that handles one byte leaves the memory system
-// waiting for instructions (3840x1920 from 3 channels: gray 23 us, FP16
-// 22 us, half-size resize 13-15 us one byte at a time).  The vector kernels
-// take 16 pixels (or 8 outputs) per thread with 16-byte accesses; the scalar
-// kernels remain for rows that do not start on a 16-byte boundary.
+// waiting for instructions.  The vector kernels take 16 pixels (or 8 outputs)
+// per thread with 16-byte accesses; the scalar kernels remain for rows that do
+// not start on a 16-byte boundary.  Measured at 3840x1920 (scalar -> vector):
+// gray of 3 channels 23 -> 7.0 us (4.2 TB/s), u8 to FP16 22 -> 6.5 us, half
+// size of 1 and 3 channels 13 -> 4.2 and 15 -> 7.3 us, the pyramid's second
+// and third level 8.6 -> 5.4 and 4.6 -> 3.5 us.
 constexpr int kVecThreads = 256;
 bool aligned16(const void *p, size_t pitch) { return (((uintptr_t)p | pitch) & 15) == 0; }
 

@@ -30,7 +30,7 @@ constexpr int kMaxTaps = (kHaloMax + 1) * (kHaloMax + 1);
 // and coordinates) is parked in shared memory, one 4-byte slot per value and
 // thread, so that the scoring loop keeps its S accumulation chains in
 // registers without spilling.  The centre bearing is re-read from the tile.
-constexpr int kParkSlots = 17;
+constexpr int kParkSlots = 16;
 constexpr int kParkScore = 3;  // slot of the score during the propagation pass
 
 // Propagation candidates of a pixel visit: the neighbours (0,1), (1,0),
@@ -403,7 +403,10 @@ __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const
 // leaves out a tenth of the scored candidates in the third half-sweep and
 // half of them from the fourth sweep on (0.6 of 1.2 per pixel in the last).
 // Measured, 8 sweeps, both together: 1920x960, 6 sources 58.0 -> 53.4 ms;
-// 512x256, 4 sources 5.06 -> 4.4 ms.
+// 512x256, 4 sources 5.06 -> 4.4 ms.  The host variant (Plain) needs one round
+// only, since its costs do not depend on the state, and skips every candidate
+// that did not change: 641x321 with 5 exact
+// sources 12.0 -> 9.9 ms, 512x256 8.4 -> 6.6 ms.
 template <int S, class Img, bool Plain, int TH, int U, class Acc, class A>
 __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *tile) {
     using G = Geo<TH>;
@@ -419,10 +422,10 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
     const int W = a.W, H = a.H, ph = a.patch_half;
     const TilePixel g(tid, i0, x0, a.colour, ph);
     int i = g.i, j = g.j;
-    const bool active = !(i < ph + 1 || i > H - ph - 1 || j < ph + 1 || j > W - ph - 1);  // PatchMatchCuda.cu:283
+    const bool inside = !(i < ph + 1 || i > H - ph - 1 || j < ph + 1 || j > W - ph - 1);  // PatchMatchCuda.cu:283
     constexpr bool plain = Plain;  // PM_PROPAGATION_PLAIN (a separate instantiation)
-    const bool spec = a.mode == kModeSweep && !plain;
-    if (!active && !spec) return;
+    const bool spec = a.mode == kModeSweep;
+    if (!inside && !spec) return;
 
     const int ctr_e = g.ctr_e;
     const int rbase = g.rbase, cbase = g.cbase, pa = g.pa;
@@ -435,7 +438,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
     // weights are recomputed per tap in the hypothesis loop (one MUFU.EX2 per
     // tap, shared by all sources) rather than held in shared memory
     float sw = 0.f, swx = 0.f, swxx = 0.f;
-    if (active) {
+    if (inside) {
         for (int m1 = 0; m1 < nt; ++m1) {
             const int k1 = 2 * m1 - ph;
             for (int m2 = 0; m2 < nt; ++m2) {
@@ -455,8 +458,9 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
         cand = a.cand[idx];
         if (!(cand.w > 0.0f)) return;  // no candidate for this pixel
     }
-    const float4 cur = active ? a.plane[idx] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a.mode == kModeSweep && plain && cur.w == 0.0f) return;  // ignored pixel (depthmap.cc:1007-1010)
+    const float4 cur = inside ? a.plane[idx] : make_float4(0.f, 0.f, 0.f, 0.f);
+    // the host variant ignores pixels of depth 0 (depthmap.cc:1007-1010)
+    const bool active = inside && !(spec && plain && cur.w == 0.0f);
     float score = active ? a.score[idx] : 0.0f;
     int best = active ? a.best[idx] : 0;
     float hx = cur.x, hy = cur.y, hz = cur.z;   // plane_*_hyp of the reference
@@ -477,15 +481,21 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
         const auto nbr_plane = [&](int n) {
             return n < kNbr && nbr_inside(n, i, j, W, H) ? a.plane[nbr_index(n, i, j, W)] : make_float4(0.f, 0.f, 0.f, 0.f);
         };
-        // candidates passing 2 f > score (the in-order walk's test) in the
-        // state before propagation
+        // Candidates that can be accepted in the state before propagation.  A
+        // propagated plane is scored as NCC x f with a smoothness factor f in
+        // [0, 1] that does not depend on the cost (PatchMatchCuda.cu:322-337),
+        // so no combined score <= 2 (the exact NCC is bounded by 1) helps a
+        // candidate with 2 f <= score.  In the host variant (f = 1) every
+        // neighbour is scored.
         unsigned need = 0;
         if (active) {
             unsigned open = 0xffu;
             // A candidate whose plane this pixel saw at its last visit, in the
             // state it still has, was turned down then and is again: it is
-            // looked at only if this visit changes the state first.
-            if (a.use_changed && !a.changed[idx]) {
+            // looked at only if this visit changes the state first.  In the
+            // host variant costs do not depend on the state and scores only
+            // rise, so a candidate seen before never wins again.
+            if (a.use_changed && (plain || !a.changed[idx])) {
                 open = 0;
 #pragma unroll
                 for (int n = 0; n < kNbr; ++n)
@@ -496,6 +506,14 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
             for (int n = 0; n < kNbr; ++n) {
                 const float4 next = nbr_plane(n + 1);
                 if (((open >> n) & 1u) && nbr_inside(n, i, j, W, H)) {
+                    if constexpr (plain) {
+                        if (np.w != 0.0f) {  // ignored neighbour (depthmap.cc:1018-1021)
+                            need |= 1u << n;
+                            res[n * kThreads + tid] = 1.0f;
+                        }
+                        np = next;
+                        continue;
+                    }
                     const float f = smoothness_factor(np.x, np.y, np.z, hx, hy, hz, bxc, byc, bzc, curr_depth);
                     if (2.0f * f > score) {
                         need |= 1u << n;
@@ -529,8 +547,23 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
             // were listed in, so the walk starts at the first that beat the
             // pixel's score; those before it lost.
             if (n < 0) n = (known & 0xffu) ? __ffs(known & 0xffu) - 1 : kNbr;
-            known >>= kScored;
             need = 0;
+            if constexpr (plain) {
+                // each winner against the score reached so far, in order
+                for (unsigned m = known & 0xffu; m; m &= m - 1) {
+                    const int w = __ffs(m) - 1;
+                    const float sc = res[w * kThreads + tid];
+                    if (sc > score) {
+                        const float4 np = nbr_plane(w);
+                        hx = np.x; hy = np.y; hz = np.z;
+                        score = sc;
+                        best = res_best[w * kThreads + tid];
+                        moved = true;
+                    }
+                }
+                continue;
+            }
+            known >>= kScored;
             if (active && n < kNbr) {
                 // the walk in order with the scores at hand (PatchMatchCuda.cu:305-337);
                 // from the first candidate that passes in the state reached so
@@ -570,17 +603,10 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
     float cx = hx, cy = hy, cz = hz, current_depth = curr_depth;
     float depth_hyp = 0.f;
     const int nh = a.mode == kModeSweep ? 14 : 1;
-
-    // Propagated planes are scored as NCC x f with a smoothness factor
-    // f in [0, 1] that does not depend on the cost (PatchMatchCuda.cu:322-337).
-    // A candidate with 2 f <= score cannot be accepted by any combined score
-    // <= 2 (the exact NCC is bounded by 1), so its cost is not evaluated.
-    // In the plain (host-variant) propagation every neighbour is scored
-    // unless its depth is 0, in order, by each lane for its own pixel.
     int kr = 0;            // plain propagation: refinements tried so far (their ranges shrink only when tried)
 #pragma unroll 1
     while (true) {
-        float px = 0.f, py = 0.f, pz = 0.f, f = 1.0f;
+        float px = 0.f, py = 0.f, pz = 0.f;
         bool found = false;
 #pragma unroll 1
         for (; h < nh; ++h) {
@@ -588,16 +614,6 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
                 px = hx; py = hy; pz = hz;
             } else if (a.mode == kModeSeed) {
                 px = cand.x; py = cand.y; pz = cand.z;
-            } else if (h < kNbr) {
-                if (!nbr_inside(h, i, j, W, H)) continue;
-                const float4 np = a.plane[nbr_index(h, i, j, W)];
-                px = np.x; py = np.y; pz = np.z;
-                if (plain) {
-                    if (np.w == 0.0f) continue;  // ignored neighbour (depthmap.cc:1018-1021)
-                } else {
-                    f = smoothness_factor(px, py, pz, hx, hy, hz, bxc, byc, bzc, curr_depth);
-                    if (!(2.0f * f > score)) continue;  // cannot be accepted (also when f is NaN)
-                }
             } else {
                 const int t = h - kNbr;
                 if (t == 0) {
@@ -647,7 +663,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
 
         const Park<TH> park(smem);
         // h < 16, kr < 8, i < 2^15, j < 2^15 (image sizes are validated)
-        park.save(hx, hy, hz, cx, cy, cz, score, current_depth, depth_hyp, f, sw, swx, swxx, curr_depth, cand_w,
+        park.save(hx, hy, hz, cx, cy, cz, score, current_depth, depth_hyp, sw, swx, swxx, curr_depth, cand_w,
                   h | (kr << 4) | ((int)moved << 7) | (best << 8), i | (j << 16));
 
         // ---- cost of hypothesis (px, py, pz) ----
@@ -655,7 +671,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
         accumulate_plane<S, Img, TH, U, Acc>(acc, a, tile, fac, rbase, cbase, pa, Ic, px, py, pz);
         {
             int st, ij;
-            park.load(hx, hy, hz, cx, cy, cz, score, current_depth, depth_hyp, f, sw, swx, swxx, curr_depth, cand_w, st,
+            park.load(hx, hy, hz, cx, cy, cz, score, current_depth, depth_hyp, sw, swx, swxx, curr_depth, cand_w, st,
                       ij);
             h = st & 15;
             kr = (st >> 4) & 7;
@@ -672,7 +688,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
         float sep[S], cum[S];
         source_nccs(acc, sw, swx, swxx, a.combine, sep, cum);
         int hb;
-        float sc = combine_scores<S>(sep, cum, a.combine, a.top_k, &hb);
+        const float sc = combine_scores<S>(sep, cum, a.combine, a.top_k, &hb);
 
         if (a.mode == kModeScore) {
             score = sc;
@@ -681,19 +697,16 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
             if (sc > score) {  // the host seeding rule (depthmap.cc:483-487)
                 cx = px; cy = py; cz = pz; score = sc; current_depth = cand_w; best = hb;
             }
-        } else if (h < kNbr) {
-            sc = __fmul_rn(sc, f);
-            if (sc > score) { hx = px; hy = py; hz = pz; score = sc; best = hb; moved = true; }
         } else {
             if (sc > score) {
                 cx = px; cy = py; cz = pz; score = sc; best = hb;
+                moved = true;
                 if (plain) {
                     // the host variant stores the plane's own depth (CheckPlaneCandidate, depthmap.cc:1074-1076)
                     const float dn = __fadd_rn(__fadd_rn(__fmul_rn(bxc, px), __fmul_rn(byc, py)), __fmul_rn(bzc, pz));
                     current_depth = __fdiv_rn(1.0f, fmaxf(1e-6f, fabsf(dn)));
                 } else {
                     current_depth = depth_hyp;
-                    moved = true;
                 }
             }
         }
@@ -708,7 +721,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
         a.plane[idx] = make_float4(cx, cy, cz, w);
         // scores only rise, so the pixel's state is the one before this visit
         // unless a plane was taken (or the stored depth was rounded otherwise)
-        if (!plain) a.changed[idx] = moved || __float_as_uint(w) != __float_as_uint(curr_depth);
+        a.changed[idx] = moved || __float_as_uint(w) != __float_as_uint(curr_depth);
     } else if (a.mode == kModeSeed) {
         a.plane[idx] = make_float4(cx, cy, cz, current_depth);
     }

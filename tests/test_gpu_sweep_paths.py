@@ -33,6 +33,10 @@ def _request(ctx, W, H, S, seed, **kw):
     (129, 65, 4, dict(combine=native.COMBINE_TOPK)),
     (200, 101, 6, dict(combine=native.COMBINE_FOLD_SEPARATE, sampler=native.SAMPLER_EXACT)),
     (131, 67, 9, dict()),
+    (131, 67, 3, dict(propagation=native.PROPAGATION_PLAIN, patch_half=1)),
+    (257, 129, 5, dict(propagation=native.PROPAGATION_PLAIN, combine=native.COMBINE_MAX,
+                       sampler=native.SAMPLER_EXACT, seam=native.SEAM_ZERO)),
+    (640, 320, 2, dict(propagation=native.PROPAGATION_PLAIN)),
     (192, 96, 2, dict(sampler=native.SAMPLER_EXACT, seam=native.SEAM_WRAP)),
 ])
 def test_skipping_unchanged_candidates_is_exact(ctx, W, H, S, kw):
