@@ -472,8 +472,8 @@ int pm_fuse_noalloc(int width, int height, int n_views, float *const *depths, co
  * CUDA graph and replayed by pm_batch_run.  Requests are grouped by source
  * count, image variant, propagation rule and sweep count; each phase of a
  * group is one persistent launch over a device queue of (request, 8x64 tile)
- * items (PM_BATCH_PERSISTENT, grid = grid_mult x resident CTAs) or one launch
- * per request (PM_BATCH_LAUNCHES); PM_BATCH_STREAMS instead runs each
+ * items (PM_BATCH_PERSISTENT, grid = grid_mult x resident CTAs, the groups on
+ * parallel graph branches) or one launch per request (PM_BATCH_LAUNCHES); PM_BATCH_STREAMS instead runs each
  * request's whole chain on one of 8 parallel graph branches (largest request
  * first onto the least-loaded branch) so that requests overlap on the GPU;
  * PM_BATCH_MIXED is one persistent launch per phase over all requests of

@@ -215,6 +215,17 @@ int validate_size(pm_ctx *ctx, int W, int H, int S) {
 
 }  // namespace
 
+long long pmi::tile_warps(const pm_request *r) {
+    return (long long)((r->W + pm::kTileWidth - 1) / pm::kTileWidth) * r->H;
+}
+
+int pmi::tile_rows(const pm_request *r, long long warps) {
+    // all tiles resident at once: the latency of one tile visit counts
+    const int max_warps = r->prm.sampler == PM_SAMPLER_TEXTURE ? kSmallWarpsTexture : kSmallWarpsQuad;
+    return r->S <= pm::kSmallMaxSources && warps <= (long long)max_warps * r->ctx->n_sm ? pm::kTileRowsSmall
+                                                                                       : pm::kTileRowsLarge;
+}
+
 int pmi::tile_band(pm_request *r, dim3 grid, cudaStream_t st, pm::BandArgs *band, const pm::BandArgs **out) {
     *out = nullptr;
     if (r->banded_blocks <= 0) return PM_OK;
@@ -362,11 +373,7 @@ int ensure_textures(pm_request *r) {
 // 4-6 % slower banded at 1920x960).
 void set_tile_order(pm_request *r) {
     r->banded_blocks = 0;
-    // all tiles resident at once: the latency of one tile visit counts
-    const int max_warps = r->prm.sampler == PM_SAMPLER_TEXTURE ? kSmallWarpsTexture : kSmallWarpsQuad;
-    const long long warps = (long long)((r->W + pm::kTileWidth - 1) / pm::kTileWidth) * r->H;
-    r->tile_rows = r->S <= pm::kSmallMaxSources && warps <= (long long)max_warps * r->ctx->n_sm ? pm::kTileRowsSmall
-                                                                                                : pm::kTileRowsLarge;
+    r->tile_rows = pmi::tile_rows(r, pmi::tile_warps(r));
     if (r->tile_rows == pm::kTileRowsSmall) return;
     if (r->ctx->n_sm <= 0 || r->ctx->n_sm > kMaxBands / 2 || r->prm.sampler != PM_SAMPLER_TEXTURE) return;
     const size_t texel = r->prm.image_format == PM_IMAGE_F16 ? 2 : 1;

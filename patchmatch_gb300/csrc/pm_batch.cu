@@ -22,8 +22,8 @@ using pmi::fill_args;
 // post-filter), captured once into a CUDA graph and replayed.  Requests are
 // grouped by (source count, image variant, propagation rule, sweep count);
 // each phase of a group is one persistent launch over a device queue of
-// (request, tile) items (PM_BATCH_PERSISTENT) or one launch per request
-// (PM_BATCH_LAUNCHES).  A tile's update reads only pixels of the other colour,
+// (request, tile) items (PM_BATCH_PERSISTENT; the groups on parallel graph
+// branches) or one launch per request (PM_BATCH_LAUNCHES).  A tile's update reads only pixels of the other colour,
 // so the result of every request is the same as from pm_request_run.
 // ---------------------------------------------------------------------------
 struct pm_batch {
@@ -160,11 +160,8 @@ int batch_enqueue(pm_batch *b) {
     int sms = 0;
     PM_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     uint64_t launches = 0;
-    int max_phases = 0;
-    for (auto &g : b->groups) {
+    for (auto &g : b->groups)
         PM_CUDA(ctx, cudaMemsetAsync(g.d_counters, 0, g.n_phases * sizeof(unsigned int), st));
-        max_phases = std::max(max_phases, g.n_phases);
-    }
     if (b->executor == PM_BATCH_STREAMS) {
         // each request's whole chain on one of the branch streams (largest
         // first onto the least-loaded branch), branches forked from and
@@ -180,6 +177,10 @@ int batch_enqueue(pm_batch *b) {
             if (b->level[x] != b->level[y]) return b->level[x] < b->level[y];
             return work(x) > work(y);
         });
+        // requests that share the device take the tile height of their sum (12
+        // requests 256 to 384 wide: 8.9 ms in large tiles, 12.0 ms in small ones)
+        long long warps = 0;
+        for (const pm_request *r : b->reqs) warps += pmi::tile_warps(r);
         double load[pm_batch::kBranches] = {};
         std::vector<int> branch_of(b->reqs.size(), -1);
         const int nb = std::min<int>(pm_batch::kBranches, (int)order.size());
@@ -213,12 +214,13 @@ int batch_enqueue(pm_batch *b) {
                 a.colour = ph < 2 ? ph : (ph - 2) & 1;
                 a.sweep = ph < 2 ? 0 : (ph - 2) >> 1;
                 a.use_changed = ph >= 4;
-                const dim3 grid = pm::tile_grid(r->W, r->H, r->tile_rows);
+                const int rows = pmi::tile_rows(r, warps);
+                const dim3 grid = pm::tile_grid(r->W, r->H, rows);
                 pm::BandArgs band{};
                 const pm::BandArgs *bp = nullptr;
                 const int rc = pmi::tile_band(r, grid, bs, &band, &bp);
                 if (rc) return rc;
-                cudaError_t e = pm::dispatch_tile(r->S, kind, r->tile_rows, grid, bs, a, bp);
+                cudaError_t e = pm::dispatch_tile(r->S, kind, rows, grid, bs, a, bp);
                 if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
                 ++launches;
             }
@@ -238,77 +240,126 @@ int batch_enqueue(pm_batch *b) {
         b->launches_per_run = launches;
         return PM_OK;
     }
-    for (int lv = 0; lv < b->n_levels; ++lv) {
-    for (size_t k = 0; k < b->reqs.size(); ++k) {
-        if (b->level[k] != lv) continue;
-        pm_request *r = b->reqs[k];
-        const pm_params &p = r->prm;
-        pm::launch_init_planes(st, r->trig.row, r->trig.col, r->W, r->H, p.seed, p.keyframe_id, p.init_mode,
-                               p.min_depth, p.max_depth, r->plane, r->score, r->best);
-        ++launches;
-    }
-    for (int ph = 0; ph < max_phases; ++ph) {
-        if (ph == 2) {
-            // seeding of this level's requests, between the init scoring and the sweeps
-            for (size_t k = 0; k < b->reqs.size(); ++k) {
-                if (b->level[k] != lv) continue;
-                const int rc = seed_in_batch(b, b->reqs[k], st, launches);
-                if (rc) return rc;
-            }
-        }
+    const bool queued = b->executor == PM_BATCH_PERSISTENT || b->executor == PM_BATCH_MIXED;
+    // one phase of a group: a persistent launch over its tile queue, or one launch per request
+    const auto group_phase = [&](pm_batch::Group &g, int ph, cudaStream_t gs) -> int {
         const int mode = ph < 2 ? pm::kModeScore : pm::kModeSweep;
         const int colour = ph < 2 ? ph : (ph - 2) & 1;
         const int sweep = ph < 2 ? 0 : (ph - 2) >> 1;
-        for (auto &g : b->groups) {
-            if (g.level != lv || ph >= g.n_phases) continue;
-            if (b->executor == PM_BATCH_PERSISTENT || b->executor == PM_BATCH_MIXED) {
-                pm::BatchArgs a{};
-                a.args = g.d_args;
-                a.items = g.d_items;
-                a.n_items = g.n_items;
-                a.counter = g.d_counters + ph;
-                a.mode = mode;
-                a.colour = colour;
-                a.sweep = sweep;
-                a.use_changed = ph >= 4;
-                const bool mixed = b->executor == PM_BATCH_MIXED;
-                const int occ = std::max(1, mixed ? pm::dispatch_batch_mixed_blocks_per_sm(g.kind, g.plain)
-                                                  : pm::dispatch_batch_blocks_per_sm(g.S, g.kind, g.plain));
-                const int blocks = std::max(1, std::min(g.n_items, b->grid_mult * occ * sms));
-                cudaError_t e = mixed ? pm::dispatch_batch_mixed(g.kind, g.plain, blocks, st, a)
-                                      : pm::dispatch_batch(g.S, g.kind, g.plain, blocks, st, a);
-                if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "batch launch: %s", cudaGetErrorString(e));
+        if (queued) {
+            pm::BatchArgs a{};
+            a.args = g.d_args;
+            a.items = g.d_items;
+            a.n_items = g.n_items;
+            a.counter = g.d_counters + ph;
+            a.mode = mode;
+            a.colour = colour;
+            a.sweep = sweep;
+            a.use_changed = ph >= 4;
+            const bool mixed = b->executor == PM_BATCH_MIXED;
+            const int occ = std::max(1, mixed ? pm::dispatch_batch_mixed_blocks_per_sm(g.kind, g.plain)
+                                              : pm::dispatch_batch_blocks_per_sm(g.S, g.kind, g.plain));
+            const int blocks = std::max(1, std::min(g.n_items, b->grid_mult * occ * sms));
+            cudaError_t e = mixed ? pm::dispatch_batch_mixed(g.kind, g.plain, blocks, gs, a)
+                                  : pm::dispatch_batch(g.S, g.kind, g.plain, blocks, gs, a);
+            if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "batch launch: %s", cudaGetErrorString(e));
+            ++launches;
+            return PM_OK;
+        }
+        for (size_t m = 0; m < g.members.size(); ++m) {
+            pm::SweepArgs a = g.h_args[m];
+            a.mode = mode;
+            a.colour = colour;
+            a.sweep = sweep;
+            a.use_changed = ph >= 4;
+            const int rows = g.members[m]->tile_rows;
+            const dim3 grid = pm::tile_grid(a.W, a.H, rows);
+            pm::BandArgs band{};
+            const pm::BandArgs *bp = nullptr;
+            const int rc = pmi::tile_band(g.members[m], grid, gs, &band, &bp);
+            if (rc) return rc;
+            cudaError_t e = pm::dispatch_tile(g.S, g.kind, rows, grid, gs, a, bp);
+            if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
+            ++launches;
+        }
+        return PM_OK;
+    };
+    // all phases of some groups of one level, phase-major, with their
+    // requests' initialisation, seeding and post-filter
+    const auto run_groups = [&](const std::vector<pm_batch::Group *> &gr, cudaStream_t gs) -> int {
+        int phases = 0;
+        for (pm_batch::Group *g : gr) {
+            phases = std::max(phases, g->n_phases);
+            for (pm_request *r : g->members) {
+                const pm_params &p = r->prm;
+                pm::launch_init_planes(gs, r->trig.row, r->trig.col, r->W, r->H, p.seed, p.keyframe_id, p.init_mode,
+                                       p.min_depth, p.max_depth, r->plane, r->score, r->best);
                 ++launches;
-            } else {
-                for (size_t m = 0; m < g.members.size(); ++m) {
-                    pm::SweepArgs a = g.h_args[m];
-                    a.mode = mode;
-                    a.colour = colour;
-                    a.sweep = sweep;
-                    a.use_changed = ph >= 4;
-                    const int rows = g.members[m]->tile_rows;
-                    const dim3 grid = pm::tile_grid(a.W, a.H, rows);
-                    pm::BandArgs band{};
-                    const pm::BandArgs *bp = nullptr;
-                    const int rc = pmi::tile_band(g.members[m], grid, st, &band, &bp);
-                    if (rc) return rc;
-                    cudaError_t e = pm::dispatch_tile(g.S, g.kind, rows, grid, st, a, bp);
-                    if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
-                    ++launches;
-                }
             }
         }
-    }
-    if (max_phases <= 2)  // no sweep phase in the batch: the seeding follows the init scoring
-        for (size_t k = 0; k < b->reqs.size(); ++k) {
-            if (b->level[k] != lv) continue;
-            const int rc = seed_in_batch(b, b->reqs[k], st, launches);
+        const auto seed = [&]() -> int {
+            for (pm_batch::Group *g : gr)
+                for (pm_request *r : g->members) {
+                    const int rc = seed_in_batch(b, r, gs, launches);
+                    if (rc) return rc;
+                }
+            return PM_OK;
+        };
+        for (int ph = 0; ph < phases; ++ph) {
+            int rc = ph == 2 ? seed() : PM_OK;  // between the init scoring and the sweeps
+            for (pm_batch::Group *g : gr)
+                if (!rc && ph < g->n_phases) rc = group_phase(*g, ph, gs);
             if (rc) return rc;
         }
-    for (size_t k = 0; k < b->reqs.size(); ++k)
-        if (b->level[k] == lv && b->reqs[k]->prm.postprocess) {
-            enqueue_post(b->reqs[k], st);
-            launches += 3;
+        if (phases <= 2) {  // no sweep phase: the seeding follows the init scoring
+            const int rc = seed();
+            if (rc) return rc;
+        }
+        for (pm_batch::Group *g : gr)
+            for (pm_request *r : g->members)
+                if (r->prm.postprocess) {
+                    enqueue_post(r, gs);
+                    launches += 3;
+                }
+        return PM_OK;
+    };
+    for (int lv = 0; lv < b->n_levels; ++lv) {
+        std::vector<pm_batch::Group *> here;
+        for (auto &g : b->groups)
+            if (g.level == lv) here.push_back(&g);
+        if (!queued || here.size() < 2) {
+            const int rc = run_groups(here, st);
+            if (rc) return rc;
+            continue;
+        }
+        // The groups of a level do not depend on each other: each runs its
+        // phases on one of the graph's branches (largest first onto the
+        // least-loaded), so that one group's tiles fill the SMs that another's
+        // last wave leaves idle.  Measured: six requests 480 to 1920 wide with
+        // 3-10 sources, 4 sweeps, 91.7 -> 83.8 ms; 12 requests 256 to 384 wide
+        // 15 -> 8.4 ms.
+        const auto work = [](const pm_batch::Group *g) {
+            double w = 0.0;
+            for (const pm_request *r : g->members) w += (double)r->W * r->H * r->S * (1 + r->prm.iterations);
+            return w;
+        };
+        std::stable_sort(here.begin(), here.end(),
+                         [&](const pm_batch::Group *x, const pm_batch::Group *y) { return work(x) > work(y); });
+        const int nb = std::min<int>(pm_batch::kBranches, (int)here.size());
+        double load[pm_batch::kBranches] = {};
+        PM_CUDA(ctx, cudaEventRecord(b->fork, st));
+        for (int k = 0; k < nb; ++k) PM_CUDA(ctx, cudaStreamWaitEvent(b->branch[k], b->fork, 0));
+        for (pm_batch::Group *g : here) {
+            int k = 0;
+            for (int q = 1; q < nb; ++q)
+                if (load[q] < load[k]) k = q;
+            load[k] += work(g);
+            const int rc = run_groups({g}, b->branch[k]);
+            if (rc) return rc;
+        }
+        for (int k = 0; k < nb; ++k) {
+            PM_CUDA(ctx, cudaEventRecord(b->join[k], b->branch[k]));
+            PM_CUDA(ctx, cudaStreamWaitEvent(st, b->join[k], 0));
         }
     }  // level
     b->launches_per_run = launches;

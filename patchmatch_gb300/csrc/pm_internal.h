@@ -138,6 +138,10 @@ PM_INTERNAL void fill_args(pm_request *r);
 PM_INTERNAL int check_views(pm_request *r);
 // Enqueue the post-filter of a request on `st` (its own stream when null).
 PM_INTERNAL int enqueue_post(pm_request *r, cudaStream_t st = nullptr);
+// Rows of warps (64 columns each) of the request's image, and the tile height
+// for `warps` such rows in flight on the device together.
+PM_INTERNAL long long tile_warps(const pm_request *r);
+PM_INTERNAL int tile_rows(const pm_request *r, long long warps);
 // The band arguments of the request's tile order for one launch of `grid`
 // on `st`, with the band counters reset there first; *out is null when the
 // request runs one CTA per tile.
