@@ -734,17 +734,19 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, tile_min_blocks<S>()) t
 }
 
 // The same visit for images whose tiles all fit the chip at once (the rule is
-// in pm_api.cu, set_tile_order).  There a half-sweep lasts as long as one
-// tile's chain of costs, so the tiles have 4 rows (twice as many SMs get one),
-// and a lane runs two taps' worth of chains side by side, in the 128 registers
-// that 16 warps per SM leave each thread (from 7 sources one tap fills them).
-// Measured, 8 sweeps, against the kernel above: 256x128 2 sources 2.08 ->
-// 1.43 ms, 4 sources 3.34 -> 2.10 ms; 448x224 4 sources 4.07 -> 3.49 ms;
-// 512x256 2 sources 3.05 -> 2.55 ms, 4 sources 4.48 -> 4.27 ms.  Tiles of 2
-// rows (4.65 ms at 512x256 with 4 sources) and 1 row (4.81 ms) lose more to
-// their halos and part-filled lists; three taps at once spill from 5 sources.
+// in pm_api.cu, tile_rows).  There a half-sweep lasts as long as one tile's
+// chain of costs, so the tiles have 4 rows (twice as many SMs get one), and a
+// lane runs the chains of several taps side by side, as many as the 128
+// registers hold that 16 warps per SM leave each thread.  Measured, 8 sweeps,
+// against the kernel above: 256x128 1 source 1.78 -> 0.95 ms, 2 sources 2.08 ->
+// 1.25 ms, 4 sources 3.34 -> 2.00 ms; 512x256 2 sources 3.05 -> 2.51 ms, 4
+// sources 4.48 -> 4.15 ms.  Taps at once at 256x128, 2 / 3 / 6: 1 source 1.25 /
+// 1.09 / 0.95 ms, 2 sources 1.49 / 1.34 / 1.25, 3 sources 1.75 / 1.67 / 1.74, 4
+// sources 2.12 / 2.00 / 2.31 (spills).  Tiles of 2 rows (4.65 ms at 512x256
+// with 4 sources) and 1 row (4.81 ms) lose more to their halos and part-filled
+// lists.
 template <int S>
-__host__ __device__ constexpr int small_taps() { return S <= 6 ? 2 : 1; }
+__host__ __device__ constexpr int small_taps() { return S <= 2 ? 6 : S <= 4 ? 3 : S <= 6 ? 2 : 1; }
 constexpr int kSmallMinBlocks = 4;
 constexpr int kSmallMaxSources = 8;  // with 9 and 10 (factored warp) 333x167 is even or 7 % slower in small tiles
 template <int S, class Img, bool Plain>
