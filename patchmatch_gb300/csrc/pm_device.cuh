@@ -269,25 +269,26 @@ __device__ __forceinline__ float bilateral_weight(float xs, float ncf, float dk)
     return exp2f(fmaf(xs * xs, ncf, dk));
 }
 
-// The three standard normals of refinement t (0..5) of one pixel visit:
-// normals 3t..3t+2 of the Box-Muller stream whose pair p uses Philox block
-// p / 2, words (x, y) for even p and (z, w) for odd p.
-__device__ __forceinline__ void refine_normals(uint32_t seed, uint32_t kf, uint32_t pix, uint32_t tag, int t,
-                                               float &ra, float &rb, float &rc) {
+// The six standard normals of refinements t and t + 1 (t even) of one pixel
+// visit: normals 3t..3t+5 of the Box-Muller stream whose pair p uses Philox
+// block p / 2, words (x, y) for even p and (z, w) for odd p.  Two refinements
+// at a time take two blocks and three pairs; one at a time took two blocks and
+// two pairs each, a third of the draws twice.
+__device__ __forceinline__ void refine_normals2(uint32_t seed, uint32_t kf, uint32_t pix, uint32_t tag, int t,
+                                                float (&z)[6]) {
     const int p0 = (3 * t) >> 1;
-    float z[4];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int p = p0 + q;
-        const uint4 blk = philox_block(seed, kf, pix, tag, (uint32_t)(p >> 1));
-        const float2 bm = (p & 1) ? box_muller(blk.z, blk.w) : box_muller(blk.x, blk.y);
-        z[2 * q] = bm.x;
-        z[2 * q + 1] = bm.y;
-    }
-    const bool odd = (3 * t) & 1;
-    ra = odd ? z[1] : z[0];
-    rb = odd ? z[2] : z[1];
-    rc = odd ? z[3] : z[2];
+    const uint4 b0 = philox_block(seed, kf, pix, tag, (uint32_t)(p0 >> 1));
+    const uint4 b1 = philox_block(seed, kf, pix, tag, (uint32_t)(p0 >> 1) + 1u);
+    const bool odd = p0 & 1;
+    const float2 n0 = box_muller(odd ? b0.z : b0.x, odd ? b0.w : b0.y);
+    const float2 n1 = box_muller(odd ? b1.x : b0.z, odd ? b1.y : b0.w);
+    const float2 n2 = box_muller(odd ? b1.z : b1.x, odd ? b1.w : b1.y);
+    z[0] = n0.x;
+    z[1] = n0.y;
+    z[2] = n1.x;
+    z[3] = n1.y;
+    z[4] = n2.x;
+    z[5] = n2.y;
 }
 
 // The four standard normals of refinement t of the plain (host-variant)
@@ -514,16 +515,24 @@ struct TapAccum {
 };
 
 // NCC from shifted moments (PatchMatchCuda.cu:161-170): -1 when either
-// weighted variance is below 0.1.
-__device__ __forceinline__ float ncc_from_moments(float sw, float swx, float swxx, float swy, float swyy,
-                                                  float swxy) {
-    const float prob = 1.0f / sw;
-    const float mx = swx * prob, my = swy * prob;
-    const float vx = fmaf(-mx, mx, swxx * prob);
-    const float vy = fmaf(-my, my, swyy * prob);
-    const float cov = fmaf(-mx, my, swxy * prob);
-    const float ncc = cov / sqrtf(vx * vy);
-    return (vx < 0.1f || vy < 0.1f) ? -1.0f : ncc;
+// weighted variance is below 0.1.  RefMoments: the reference window's part,
+// the same for every source.
+struct RefMoments {
+    float prob, mx, vx;
+    __device__ __forceinline__ RefMoments(float sw, float swx, float swxx)
+        : prob(1.0f / sw), mx(swx * prob), vx(fmaf(-mx, mx, swxx * prob)) {}
+};
+struct SrcMoments {
+    float vy, cov;
+    __device__ __forceinline__ SrcMoments(const RefMoments &x, float swy, float swyy, float swxy) {
+        const float my = swy * x.prob;
+        vy = fmaf(-my, my, swyy * x.prob);
+        cov = fmaf(-x.mx, my, swxy * x.prob);
+    }
+};
+__device__ __forceinline__ float ncc_of(const RefMoments &x, const SrcMoments &y) {
+    const float ncc = y.cov / sqrtf(x.vx * y.vy);
+    return (x.vx < 0.1f || y.vy < 0.1f) ? -1.0f : ncc;
 }
 
 // View combination; best = argmax of the per-source NCCs (sep).
@@ -547,30 +556,28 @@ __device__ __forceinline__ float fold_scores(const float (&v)[S]) {
 }
 
 template <int S>
-__device__ __forceinline__ float combine_scores(const float (&sep)[S], const float (&cum)[S], int mode, int top_k,
-                                                int *best) {
+__device__ __forceinline__ int argmax(const float (&v)[S]) {
     int b = 0;
+    float m = v[0];
 #pragma unroll
-    for (int r = 1; r < S; ++r) b = (sep[r] > sep[b]) ? r : b;
-    *best = b;
-    if (mode == PM_COMBINE_FOLD) return fold_scores<S>(cum);
-    if (mode == PM_COMBINE_FOLD_SEPARATE) return fold_scores<S>(sep);
-    if (mode == PM_COMBINE_MAX) {
-        float m = sep[0];
-#pragma unroll
-        for (int r = 1; r < S; ++r) m = fmaxf(m, sep[r]);
-        return m;
+    for (int r = 1; r < S; ++r) {
+        b = v[r] > m ? r : b;
+        m = v[r] > m ? v[r] : m;
     }
-    // PM_COMBINE_TOPK: sum of the k largest by repeated selection
+    return b;
+}
+
+// PM_COMBINE_TOPK: mean of the k largest by repeated selection, summed in
+// descending order.
+template <int S>
+__device__ __forceinline__ float top_mean(const float (&sep)[S], int top_k) {
     float v[S];
 #pragma unroll
     for (int r = 0; r < S; ++r) v[r] = sep[r];
     const int k = top_k < 1 ? 1 : (top_k > S ? S : top_k);
-    float accf = 0.0f;  // summed in descending order
+    float accf = 0.0f;
     for (int a = 0; a < k; ++a) {
-        int bi = 0;
-#pragma unroll
-        for (int r = 1; r < S; ++r) bi = (v[r] > v[bi]) ? r : bi;
+        const int bi = argmax<S>(v);
         float m = v[0];
 #pragma unroll
         for (int r = 0; r < S; ++r) m = (r == bi) ? v[r] : m;
@@ -581,13 +588,65 @@ __device__ __forceinline__ float combine_scores(const float (&sep)[S], const flo
     return accf / (float)k;
 }
 
-// Per-source and cumulative NCCs of one hypothesis from the window moments.
+// Per-source NCCs of one hypothesis from the window moments.
 template <int S, class Img, class Acc>
-__device__ __forceinline__ void source_nccs(const TapAccum<S, Img, Acc> &acc, float sw, float swx, float swxx, int mode,
-                                            float (&sep)[S], float (&cum)[S]) {
+__device__ __forceinline__ void source_nccs(const TapAccum<S, Img, Acc> &acc, float sw, float swx, float swxx,
+                                            float (&sep)[S]) {
+    const RefMoments x(sw, swx, swxx);
 #pragma unroll
-    for (int r = 0; r < S; ++r) sep[r] = ncc_from_moments(sw, swx, swxx, acc.swy(r), acc.swyy(r), acc.swxy(r));
-    if (mode == PM_COMBINE_FOLD) {
+    for (int r = 0; r < S; ++r) sep[r] = ncc_of(x, SrcMoments(x, acc.swy(r), acc.swyy(r), acc.swxy(r)));
+}
+
+// Combined score of one hypothesis from the window moments, and its best
+// source.  The fold over accumulated moments and the maximum need the
+// per-source NCCs only for the best source, so those are ranked by
+// cov * rsqrt(vx vy): that is within 1e-6 of the NCC, relatively, so a lead of
+// more than 1e-5 decides, and closer races (ties among them) are settled by
+// the NCCs themselves.  A square root and a division per source fall away.
+template <int S, class Img, class Acc>
+__device__ __forceinline__ float score_moments(const TapAccum<S, Img, Acc> &acc, float sw, float swx, float swxx,
+                                               int mode, int top_k, int *best) {
+    if (mode == PM_COMBINE_FOLD || mode == PM_COMBINE_MAX) {
+        const RefMoments x(sw, swx, swxx);
+        float v[S];
+#pragma unroll
+        for (int r = 0; r < S; ++r) {
+            const SrcMoments y(x, acc.swy(r), acc.swyy(r), acc.swxy(r));
+            v[r] = y.vy < 0.1f ? -1.0f : y.cov * rsqrtf(x.vx * y.vy);
+        }
+        int b = argmax<S>(v);
+        float top = v[0], next = -3.0e38f;
+#pragma unroll
+        for (int r = 1; r < S; ++r) {
+            next = fmaxf(next, fminf(top, v[r]));
+            top = fmaxf(top, v[r]);
+        }
+        if (x.vx < 0.1f) {
+            b = 0;  // every NCC is -1
+        } else if (!(v[0] == v[0] && top - next > 1e-5f * fmaxf(1.0f, fabsf(top)))) {
+            float sep[S];
+            source_nccs(acc, sw, swx, swxx, sep);
+            b = argmax<S>(sep);
+            if (mode == PM_COMBINE_MAX) {
+                float m = sep[0];
+#pragma unroll
+                for (int r = 1; r < S; ++r) m = fmaxf(m, sep[r]);
+                *best = b;
+                return m;
+            }
+        }
+        *best = b;
+        if (mode == PM_COMBINE_MAX) {
+            float y = 0.f, yy = 0.f, xy = 0.f;
+#pragma unroll
+            for (int r = 0; r < S; ++r) {
+                y = r == b ? acc.swy(r) : y;
+                yy = r == b ? acc.swyy(r) : yy;
+                xy = r == b ? acc.swxy(r) : xy;
+            }
+            return ncc_of(x, SrcMoments(x, y, yy, xy));
+        }
+        float cum[S];
         float cy = 0.f, cyy = 0.f, cxy = 0.f;
 #pragma unroll
         for (int r = 0; r < S; ++r) {
@@ -595,12 +654,15 @@ __device__ __forceinline__ void source_nccs(const TapAccum<S, Img, Acc> &acc, fl
             cyy += acc.swyy(r);
             cxy += acc.swxy(r);
             const float n = (float)(r + 1);
-            cum[r] = ncc_from_moments(n * sw, n * swx, n * swxx, cy, cyy, cxy);
+            const RefMoments xn(n * sw, n * swx, n * swxx);
+            cum[r] = ncc_of(xn, SrcMoments(xn, cy, cyy, cxy));
         }
-    } else {
-#pragma unroll
-        for (int r = 0; r < S; ++r) cum[r] = sep[r];
+        return fold_scores<S>(cum);
     }
+    float sep[S];
+    source_nccs(acc, sw, swx, swxx, sep);
+    *best = argmax<S>(sep);
+    return mode == PM_COMBINE_FOLD_SEPARATE ? fold_scores<S>(sep) : top_mean<S>(sep, top_k);
 }
 
 }  // namespace pm

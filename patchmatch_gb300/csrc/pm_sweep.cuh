@@ -361,10 +361,9 @@ __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const
             e = list[q];
             p = e >> 3;
             n = e & 7;
-            float sep[S], cum[S];
-            source_nccs(acc, mom[p], mom[kThreads + p], mom[2 * kThreads + p], a.combine, sep, cum);
             int hb;
-            const float raw = combine_scores<S>(sep, cum, a.combine, a.top_k, &hb);
+            const float raw =
+                score_moments(acc, mom[p], mom[kThreads + p], mom[2 * kThreads + p], a.combine, a.top_k, &hb);
             const float f = res[n * kThreads + p];
             res[n * kThreads + p] = raw;
             res_best[n * kThreads + p] = (int8_t)hb;
@@ -644,8 +643,14 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
                     px = __fdiv_rn(nhx, den); py = __fdiv_rn(nhy, den); pz = __fdiv_rn(nhz, den);
                 } else {
                     // refinement t (PatchMatchCuda.cu:364-382) with Philox normals (tag sweep + 1)
-                    float ra, rb, rc;
-                    refine_normals(a.seed, a.keyframe, (uint32_t)idx, (uint32_t)(a.sweep + 1), t, ra, rb, rc);
+                    // the second of two draws waits in hx, hy, hz (free since t = 0)
+                    float ra = hx, rb = hy, rc = hz;
+                    if (!(t & 1)) {
+                        float z[6];
+                        refine_normals2(a.seed, a.keyframe, (uint32_t)idx, (uint32_t)(a.sweep + 1), t, z);
+                        ra = z[0]; rb = z[1]; rc = z[2];
+                        hx = z[3]; hy = z[4]; hz = z[5];
+                    }
                     depth_hyp = __fmul_rn(current_depth, expf(__fmul_rn(a.depth_range[t], ra)));
                     const float nr = a.normal_range[t];
                     const float nhx = __fadd_rn(cx, __fmul_rn(nr, ra));
@@ -685,10 +690,8 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
             bzc = c.z;
         }
         idx = (size_t)i * W + j;
-        float sep[S], cum[S];
-        source_nccs(acc, sw, swx, swxx, a.combine, sep, cum);
         int hb;
-        const float sc = combine_scores<S>(sep, cum, a.combine, a.top_k, &hb);
+        const float sc = score_moments(acc, sw, swx, swxx, a.combine, a.top_k, &hb);
 
         if (a.mode == kModeScore) {
             score = sc;
@@ -858,13 +861,14 @@ __global__ void __launch_bounds__(256, 2) hyp_kernel(const __grid_constant__ Hyp
             acc.add_trig(a.P, a.src, scale, half, shift, px, py, pz, rt, ct, w, xs);
         }
     }
-    float sep[S], cum[S];
-    source_nccs(acc, sw, swx, swxx, a.combine, sep, cum);
-    if (a.per_source)
+    if (a.per_source) {
+        float sep[S];
+        source_nccs(acc, sw, swx, swxx, sep);
 #pragma unroll
         for (int r = 0; r < S; ++r) a.per_source[(size_t)h * S + r] = sep[r];
+    }
     int hb;
-    const float sc = combine_scores<S>(sep, cum, a.combine, a.top_k, &hb);
+    const float sc = score_moments(acc, sw, swx, swxx, a.combine, a.top_k, &hb);
     if (a.scores) a.scores[h] = sc;
     if (a.best) a.best[h] = hb;
 }
