@@ -440,6 +440,13 @@ struct TapAccum {
     template <class MB>
     __device__ __forceinline__ void add_rot(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half, float shift,
                                             float as, MB mb, float w, float xs) {
+        typename Img::Raw raw[S];
+        fetch(P, src, scale, half, as, mb, raw);
+        add(raw, shift, w, xs);
+    }
+    template <class MB>
+    __device__ __forceinline__ static void fetch(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half,
+                                                 float as, MB mb, typename Img::Raw (&raw)[S]) {
         // phase 1: all S sample coordinates, so the S footprint loads issue
         // back to back; phase 2: bilinear + moments as they arrive
         f32x2 uv[S];
@@ -452,28 +459,29 @@ struct TapAccum {
             const float Z = fmaf(as, Acc::val(P.G[r][2].w), m.z);
             uv[r] = sample_coords<Img::kBound>(XY.x, XY.y, Z, scale, half);
         }
-        typename Img::Raw raw[S];
 #pragma unroll
         for (int r = 0; r < S; ++r) {
             const float2 c = unpack2(uv[r]);
             raw[r] = Img::fetch(Acc::ptr(src.quad[r]), Acc::tex(src.tex[r]), src.qpitch, c.x, c.y);
         }
+    }
+    __device__ __forceinline__ void add(const typename Img::Raw (&raw)[S], float shift, float w, float xs) {
         const f32x2 w2 = pack2(w, w), xs2 = pack2(xs, xs);
 #pragma unroll
-        for (int k = 0; k < kPairs; ++k) {
-            const f32x2 y = Img::centred2(raw[2 * k], raw[2 * k + 1], shift);
-            const f32x2 wy = mul2(w2, y);
-            py[k] = add2(py[k], wy);
-            pyy[k] = fma2(wy, y, pyy[k]);
-            pxy[k] = fma2(wy, xs2, pxy[k]);
-        }
-        if constexpr (S & 1) {
-            const float y = Img::centred(raw[S - 1], shift);
-            const float wy = w * y;
-            oy += wy;
-            oyy = fmaf(wy, y, oyy);
-            oxy = fmaf(wy, xs, oxy);
-        }
+        for (int k = 0; k < kPairs; ++k) add_pair(k, Img::centred2(raw[2 * k], raw[2 * k + 1], shift), w2, xs2);
+        if constexpr (S & 1) add_odd(Img::centred(raw[S - 1], shift), w, xs);
+    }
+    __device__ __forceinline__ void add_pair(int k, f32x2 y, f32x2 w2, f32x2 xs2) {
+        const f32x2 wy = mul2(w2, y);
+        py[k] = add2(py[k], wy);
+        pyy[k] = fma2(wy, y, pyy[k]);
+        pxy[k] = fma2(wy, xs2, pxy[k]);
+    }
+    __device__ __forceinline__ void add_odd(float y, float w, float xs) {
+        const float wy = w * y;
+        oy += wy;
+        oyy = fmaf(wy, y, oyy);
+        oxy = fmaf(wy, xs, oxy);
     }
     // One tap with bearing b = (bx, by, bz), rotated per source directly.
     __device__ __forceinline__ void add_bearing(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half,
@@ -487,29 +495,36 @@ struct TapAccum {
                 [&](int r) { return rotate(Acc::row(P.G[r][0]), Acc::row(P.G[r][1]), Acc::row(P.G[r][2]), bx2, by2, bz2); },
                 w, xs);
     }
-    // One tap at the grid point with row trig rt = (cos lat, sin lat) and
-    // column trig ct = (sin lon, cos lon): the factored form when
-    // factored_warp<S>() (the arithmetic of the staged tile factors), the
-    // direct rotation of the bearing otherwise; the bearing is
-    // (cos lat sin lon, -sin lat, cos lat cos lon), as in the staged tile.
-    __device__ __forceinline__ void add_trig(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half, float shift,
-                                             float px, float py_, float pz, float2 rt, float2 ct, float w, float xs) {
+    // The footprints of the tap at the grid point with row trig rt = (cos lat,
+    // sin lat) and column trig ct = (sin lon, cos lon): the factored form when
+    // factored_warp<S>() (the arithmetic of the staged tile factors), the direct
+    // rotation of the bearing otherwise; the bearing is (cos lat sin lon,
+    // -sin lat, cos lat cos lon), as in the staged tile.
+    __device__ __forceinline__ static void fetch_trig(const PmPoses &P, const SrcSet &src, f32x2 scale, f32x2 half,
+                                                      float px, float py_, float pz, float2 rt, float2 ct,
+                                                      typename Img::Raw (&raw)[S]) {
         const float bx = rt.x * ct.x, by = -rt.y, bz = rt.x * ct.y;
+        const float s = fmaf(px, bx, fmaf(py_, by, pz * bz));
+        const uint32_t sg = __float_as_uint(s) & 0x80000000u;
         if constexpr (factored_warp<S>()) {
-            const float s = fmaf(px, bx, fmaf(py_, by, pz * bz));
-            const uint32_t sg = __float_as_uint(s) & 0x80000000u;
             const float sc = flip_sign(rt.x, sg);
-            add_rot(P, src, scale, half, shift, fabsf(s),
-                    [&](int r) {
-                        const float4 g0 = Acc::row(P.G[r][0]), g1 = Acc::row(P.G[r][1]), g2 = Acc::row(P.G[r][2]);
-                        const float3 A = col_factor(g0, g1, g2, ct.x, ct.y);
-                        const float3 B = row_factor(g0, g1, g2, rt.y);
-                        return Rotated{pack2(fmaf(sc, A.x, flip_sign(B.x, sg)), fmaf(sc, A.y, flip_sign(B.y, sg))),
-                                       fmaf(sc, A.z, flip_sign(B.z, sg))};
-                    },
-                    w, xs);
+            fetch(P, src, scale, half, fabsf(s),
+                  [&](int r) {
+                      const float4 g0 = Acc::row(P.G[r][0]), g1 = Acc::row(P.G[r][1]), g2 = Acc::row(P.G[r][2]);
+                      const float3 A = col_factor(g0, g1, g2, ct.x, ct.y);
+                      const float3 B = row_factor(g0, g1, g2, rt.y);
+                      return Rotated{pack2(fmaf(sc, A.x, flip_sign(B.x, sg)), fmaf(sc, A.y, flip_sign(B.y, sg))),
+                                     fmaf(sc, A.z, flip_sign(B.z, sg))};
+                  },
+                  raw);
         } else {
-            add_bearing(P, src, scale, half, shift, px, py_, pz, bx, by, bz, w, xs);
+            const float sbx = flip_sign(bx, sg), sby = flip_sign(by, sg), sbz = flip_sign(bz, sg);
+            const f32x2 bx2 = pack2(sbx, sbx), by2 = pack2(sby, sby), bz2 = pack2(sbz, sbz);
+            fetch(P, src, scale, half, fabsf(s),
+                  [&](int r) {
+                      return rotate(Acc::row(P.G[r][0]), Acc::row(P.G[r][1]), Acc::row(P.G[r][2]), bx2, by2, bz2);
+                  },
+                  raw);
         }
     }
 };

@@ -81,7 +81,7 @@ int banded_occ() {
 }
 template <class Img>
 cudaError_t hyp_launch(int n, cudaStream_t st, const HypArgs &a) {
-    hyp_kernel<PM_INST_S, Img><<<(n + 255) / 256, 256, 0, st>>>(a);
+    hyp_kernel<PM_INST_S, Img><<<(n + kHypThreads - 1) / kHypThreads, kHypThreads, 0, st>>>(a);
     return cudaGetLastError();
 }
 

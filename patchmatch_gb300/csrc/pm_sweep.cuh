@@ -829,38 +829,75 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S
     }
 }
 
-// Fixed-hypothesis scoring: one thread per (pixel, plane); taps read straight
-// from global memory (L1-resident) instead of a staged tile.  Same per-tap
-// arithmetic (TapAccum) as the tile kernel.
+// Fixed-hypothesis scoring, a warp for 32 (pixel, plane) pairs, with the per-tap
+// arithmetic of the tile kernel (TapAccum).  The lanes sample a row of taps of
+// all 32 side by side, lane e the tap e % taps of hypothesis e / taps, so that
+// one load covers five or six hypotheses, each with the adjacent footprints of
+// one row.  The samples pass through shared memory to the hypothesis' own
+// lane, which adds them up in the taps' order.
+// Bound by the footprints' sectors, at unrelated places: with one lane per
+// hypothesis each load opened 32 of them per source, and a sector had left the
+// L1 before the next tap came for it.  500,000 hypotheses with 8 sources,
+// 3840x1920: FP16 texture 1.90 -> 0.58 ms, FP16 footprints 1.06 -> 0.78,
+// u8 texture 1.04 -> 0.48; 1920x960 FP16 texture 1.05 -> 0.38.  (Scoring against
+// two or four sources at a time, which then stay in L2, and combining in a second
+// kernel gains only from 5760x2880 FP16: 0.91 -> 0.73.)
 template <int S, class Img>
-__global__ void __launch_bounds__(256, 2) hyp_kernel(const __grid_constant__ HypArgs a) {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= a.n) return;
+__global__ void __launch_bounds__(kHypThreads, 4) hyp_kernel(const __grid_constant__ HypArgs a) {
+    const int own = blockIdx.x * kHypThreads + threadIdx.x;
+    if ((own & ~31) >= a.n) return;
+    constexpr int kPitch = kHaloMax + 2;  // taps of a row, and odd: no bank conflicts
+    __shared__ float smem[kHypThreads / 32][S + 1][32 * kPitch];
+    float(*buf)[32 * kPitch] = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    // a warp's lanes work on each other's hypotheses: those past the end stay
+    const int h = min(own, a.n - 1);
     const int2 ij = a.ij[h];
-    const int i = ij.x, j = ij.y, W = a.W, ph = a.patch_half;
-    const float Ic = a.ref[(size_t)i * W + j];
-    const float px = a.planes[3 * h], py = a.planes[3 * h + 1], pz = a.planes[3 * h + 2];
-    const float shift = Img::shift_for(Ic);
+    const int W = a.W, ph = a.patch_half, nt = ph + 1;  // 2, 4 or 6 taps a row
+    const unsigned inv = 65536u / nt + 1u;              // e / nt = e * inv >> 16 for e < 32 nt
+    const float Ic = a.ref[(size_t)ij.x * W + ij.y];
+    const float px = a.planes[3 * (size_t)h], py = a.planes[3 * (size_t)h + 1], pz = a.planes[3 * (size_t)h + 2];
     const f32x2 scale = pack2(a.Wf, 2.0f * a.Hf);
     const f32x2 half = pack2(fmaf(0.5f, a.Wf, Img::kCoordOffset), fmaf(0.5f, a.Hf, Img::kCoordOffset));
     float sw = 0.f, swx = 0.f, swxx = 0.f;
     TapAccum<S, Img> acc;
     acc.zero();
     for (int k1 = -ph; k1 <= ph; k1 += 2) {
-        const int R = i + k1;
-        const float2 rt = a.row_trig[R];
-        for (int k2 = -ph; k2 <= ph; k2 += 2) {
-            const int C = j + k2;
-            const float2 ct = a.col_trig[C];
-            const float x = a.ref[(size_t)R * W + C];
-            const float xs = x - Ic;
+#pragma unroll 1
+        for (int e = lane; e < 32 * nt; e += 32) {
+            const int q = (int)(e * inv >> 16), t = e - q * nt;
+            const int R = __shfl_sync(~0u, ij.x, q) + k1, C = __shfl_sync(~0u, ij.y, q) + 2 * t - ph;
+            const float qx = __shfl_sync(~0u, px, q), qy = __shfl_sync(~0u, py, q), qz = __shfl_sync(~0u, pz, q);
+            const float qc = __shfl_sync(~0u, Ic, q);
+            typename Img::Raw raw[S];
+            TapAccum<S, Img>::fetch_trig(a.P, a.src, scale, half, qx, qy, qz, a.row_trig[R], a.col_trig[C], raw);
+            const float shift = Img::shift_for(qc);
+            const int at = q * kPitch + t;
+            buf[S][at] = a.ref[(size_t)R * W + C] - qc;
+#pragma unroll
+            for (int k = 0; k < S / 2; ++k) {
+                const float2 v = unpack2(Img::centred2(raw[2 * k], raw[2 * k + 1], shift));
+                buf[2 * k][at] = v.x;
+                buf[2 * k + 1][at] = v.y;
+            }
+            if constexpr (S & 1) buf[S - 1][at] = Img::centred(raw[S - 1], shift);
+        }
+        __syncwarp();
+        for (int t = 0; t < nt; ++t) {
+            const int at = lane * kPitch + t, k2 = 2 * t - ph;
+            const float xs = buf[S][at];
             const float w = bilateral_weight(xs, a.ncf, fmaf((float)(k2 * k2), a.ndf, (float)(k1 * k1) * a.ndf));
             sw += w;
             swx = fmaf(w, xs, swx);
             swxx = fmaf(w * xs, xs, swxx);
-            acc.add_trig(a.P, a.src, scale, half, shift, px, py, pz, rt, ct, w, xs);
+            const f32x2 w2 = pack2(w, w), xs2 = pack2(xs, xs);
+#pragma unroll
+            for (int k = 0; k < S / 2; ++k) acc.add_pair(k, pack2(buf[2 * k][at], buf[2 * k + 1][at]), w2, xs2);
+            if constexpr (S & 1) acc.add_odd(buf[S - 1][at], w, xs);
         }
+        __syncwarp();
     }
+    if (own >= a.n) return;
     if (a.per_source) {
         float sep[S];
         source_nccs(acc, sw, swx, swxx, sep);

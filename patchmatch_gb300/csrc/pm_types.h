@@ -106,5 +106,6 @@ struct HypArgs {
     int *best;            // n
     float *per_source;    // n x S or null
 };
+constexpr int kHypThreads = 128;
 
 }  // namespace pm
