@@ -150,6 +150,12 @@ __device__ __forceinline__ float interp_depth(const float *img, int W, int H, fl
 }
 
 // DepthmapCleaner::Clean (depthmap.cc:1337-1373) for every pixel of view 0.
+// Bound by the instructions of the projections and their inverses (some 470
+// a view and warp, 90 % issue-active), so a pixel stops at the view that
+// settles it: 3840x1920 with 5 views, 2 needed, 401 -> 246 us where 98 % are
+// kept; 405 -> 400 us with 3 needed and noise that leaves 59 %.  (Packing a
+// block's open pixels before each view gave 241 and 383 us, and cost small
+// maps 10 %.)
 __global__ void clean_kernel(const __grid_constant__ CleanArgs a) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= a.H || j >= a.W) return;
@@ -162,7 +168,8 @@ __global__ void clean_kernel(const __grid_constant__ CleanArgs a) {
         const float Xc = d * rt.x * ct.x, Yc = -d * rt.y, Zc = d * rt.x * ct.y;
         const float Wf = (float)a.W, Hf = (float)a.H;
         int consistent = 1;
-        for (int k = 1; k < a.n; ++k) {
+        // until the views left cannot change the outcome
+        for (int k = 1; k < a.n && consistent < a.min_consistent && consistent + a.n - k >= a.min_consistent; ++k) {
             const float *M = a.M[k], *c = a.c[k];
             const float X = M[0] * Xc + M[1] * Yc + M[2] * Zc + c[0];
             const float Y = M[3] * Xc + M[4] * Yc + M[5] * Zc + c[1];
