@@ -2,17 +2,17 @@
 // PatchMatchCuda.cu:255-270) or performs one red/black half-sweep of
 // propagation + random refinement (PatchMatchCuda.cu:273-407).
 //
-// Layout: a CTA of 256 threads owns an 8-row x 64-column image tile and
-// updates its 256 pixels of the active colour (one warp per row, one lane per
-// pixel).  All window taps of a pixel of colour c are themselves pixels of
-// colour c, so the CTA stages only those: an 18 x 37 shared-memory tile of
-// (bearing, intensity) float4 including the 5-pixel halo, indexed so that the
-// 32 lanes of a warp read 32 consecutive entries.  The hypothesis-independent
-// reference moments are computed once per visit; the inner loop then
-// evaluates each hypothesis over the 36 taps and S sources with S independent
-// accumulation chains (recomputing each tap's bilateral weight, one MUFU.EX2
-// shared by the sources).  From 9 sources the CTA also stages the row and
-// column factors of the warp (see stage_factors).
+// Layout (tile_kernel_small has four rows): a CTA of 256 threads owns an 8-row
+// x 64-column image tile and updates its 256 pixels of the active colour (one
+// warp per row, one lane per pixel).  All window taps of a pixel of colour c
+// are themselves pixels of colour c, so the CTA stages only those: an 18 x 37
+// shared-memory tile of (bearing, intensity) float4 including the 5-pixel halo,
+// indexed so that the 32 lanes of a warp read 32 consecutive entries.  The
+// hypothesis-independent reference moments are computed once per visit; the
+// inner loop then evaluates each hypothesis over the 36 taps and S sources with
+// S independent accumulation chains (recomputing each tap's bilateral weight,
+// one MUFU.EX2 shared by the sources).  From 9 sources the CTA also stages the
+// row and column factors of the warp (see stage_factors).
 #pragma once
 
 #include "pm_device.cuh"
@@ -404,8 +404,8 @@ __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const
 // Measured, 8 sweeps, both together: 1920x960, 6 sources 58.0 -> 53.4 ms;
 // 512x256, 4 sources 5.06 -> 4.4 ms.  The host variant (Plain) needs one round
 // only, since its costs do not depend on the state, and skips every candidate
-// that did not change: 641x321 with 5 exact
-// sources 12.0 -> 9.9 ms, 512x256 8.4 -> 6.6 ms.
+// that did not change: 5 exact sources,
+// 641x321 12.0 -> 9.9 ms, 512x256 8.4 -> 6.6 ms.
 template <int S, class Img, bool Plain, int TH, int U, class Acc, class A>
 __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *tile) {
     using G = Geo<TH>;
