@@ -154,6 +154,24 @@ int seed_in_batch(pm_batch *b, pm_request *r, cudaStream_t st, uint64_t &launche
     return rc;
 }
 
+// Fork the first n branches from the batch stream.
+int fork_branches(pm_batch *b, int n) {
+    PM_CUDA(b->ctx, cudaEventRecord(b->fork, b->stream));
+    for (int k = 0; k < n; ++k) PM_CUDA(b->ctx, cudaStreamWaitEvent(b->branch[k], b->fork, 0));
+    return PM_OK;
+}
+
+// Join the first n branches back, whether or not their work could be enqueued
+// (rc): a capture whose branches are not joined cannot be ended.
+int join_branches(pm_batch *b, int n, int rc) {
+    for (int k = 0; k < n; ++k) {
+        cudaError_t e = cudaEventRecord(b->join[k], b->branch[k]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->join[k], 0);
+        if (e != cudaSuccess && !rc) rc = fail(b->ctx, PM_ECUDA, "batch branch join: %s", cudaGetErrorString(e));
+    }
+    return rc;
+}
+
 int batch_enqueue(pm_batch *b) {
     pm_ctx *ctx = b->ctx;
     const cudaStream_t st = b->stream;
@@ -184,21 +202,8 @@ int batch_enqueue(pm_batch *b) {
         double load[pm_batch::kBranches] = {};
         std::vector<int> branch_of(b->reqs.size(), -1);
         const int nb = std::min<int>(pm_batch::kBranches, (int)order.size());
-        PM_CUDA(ctx, cudaEventRecord(b->fork, st));
-        for (int k = 0; k < nb; ++k) PM_CUDA(ctx, cudaStreamWaitEvent(b->branch[k], b->fork, 0));
-        for (int idx : order) {
-            pm_request *r = b->reqs[idx];
-            const int pi = r->prior ? batch_index(b, r->prior) : -1;
-            int k = 0;
-            if (pi >= 0) {
-                k = branch_of[pi];
-            } else {
-                for (int q = 1; q < nb; ++q)
-                    if (load[q] < load[k]) k = q;
-            }
-            branch_of[idx] = k;
-            load[k] += work(idx);
-            const cudaStream_t bs = b->branch[k];
+        // a request's whole chain on stream bs
+        const auto chain = [&](pm_request *r, cudaStream_t bs) -> int {
             const pm_params &p = r->prm;
             pm::launch_init_planes(bs, r->trig.row, r->trig.col, r->W, r->H, p.seed, p.keyframe_id, p.init_mode,
                                    p.min_depth, p.max_depth, r->plane, r->score, r->best);
@@ -232,11 +237,26 @@ int batch_enqueue(pm_batch *b) {
                 enqueue_post(r, bs);
                 launches += 3;
             }
+            return PM_OK;
+        };
+        int rc = fork_branches(b, nb);
+        for (int idx : order) {
+            if (rc) break;
+            const pm_request *r = b->reqs[idx];
+            const int pi = r->prior ? batch_index(b, r->prior) : -1;
+            int k = 0;
+            if (pi >= 0) {
+                k = branch_of[pi];
+            } else {
+                for (int q = 1; q < nb; ++q)
+                    if (load[q] < load[k]) k = q;
+            }
+            branch_of[idx] = k;
+            load[k] += work(idx);
+            rc = chain(b->reqs[idx], b->branch[k]);
         }
-        for (int k = 0; k < nb; ++k) {
-            PM_CUDA(ctx, cudaEventRecord(b->join[k], b->branch[k]));
-            PM_CUDA(ctx, cudaStreamWaitEvent(st, b->join[k], 0));
-        }
+        rc = join_branches(b, nb, rc);
+        if (rc) return rc;
         b->launches_per_run = launches;
         return PM_OK;
     }
@@ -347,20 +367,17 @@ int batch_enqueue(pm_batch *b) {
                          [&](const pm_batch::Group *x, const pm_batch::Group *y) { return work(x) > work(y); });
         const int nb = std::min<int>(pm_batch::kBranches, (int)here.size());
         double load[pm_batch::kBranches] = {};
-        PM_CUDA(ctx, cudaEventRecord(b->fork, st));
-        for (int k = 0; k < nb; ++k) PM_CUDA(ctx, cudaStreamWaitEvent(b->branch[k], b->fork, 0));
+        int rc = fork_branches(b, nb);
         for (pm_batch::Group *g : here) {
+            if (rc) break;
             int k = 0;
             for (int q = 1; q < nb; ++q)
                 if (load[q] < load[k]) k = q;
             load[k] += work(g);
-            const int rc = run_groups({g}, b->branch[k]);
-            if (rc) return rc;
+            rc = run_groups({g}, b->branch[k]);
         }
-        for (int k = 0; k < nb; ++k) {
-            PM_CUDA(ctx, cudaEventRecord(b->join[k], b->branch[k]));
-            PM_CUDA(ctx, cudaStreamWaitEvent(st, b->join[k], 0));
-        }
+        rc = join_branches(b, nb, rc);
+        if (rc) return rc;
     }  // level
     b->launches_per_run = launches;
     return PM_OK;
@@ -488,6 +505,7 @@ int pm_batch_run(pm_batch *b) {
         rc = batch_enqueue(b);
         cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
         ctx->launches = before;
+        if (rc || ce != cudaSuccess) cudaGetLastError();  // reported here, not by the next call's launch check
         if (rc) {
             if (g) cudaGraphDestroy(g);
             return rc;
