@@ -81,7 +81,16 @@ int banded_occ() {
 }
 template <class Img>
 cudaError_t hyp_launch(int n, cudaStream_t st, const HypArgs &a) {
-    hyp_kernel<PM_INST_S, Img><<<(n + kHypThreads - 1) / kHypThreads, kHypThreads, 0, st>>>(a);
+    const int blocks = (n + kHypThreads - 1) / kHypThreads;
+    if constexpr (PM_INST_S == 1) {  // rows unrolled: see hyp_kernel
+        switch (a.patch_half) {
+            case 1: hyp_kernel<PM_INST_S, Img, 2><<<blocks, kHypThreads, 0, st>>>(a); break;
+            case 3: hyp_kernel<PM_INST_S, Img, 4><<<blocks, kHypThreads, 0, st>>>(a); break;
+            default: hyp_kernel<PM_INST_S, Img, 6><<<blocks, kHypThreads, 0, st>>>(a); break;
+        }
+    } else {
+        hyp_kernel<PM_INST_S, Img, 0><<<blocks, kHypThreads, 0, st>>>(a);
+    }
     return cudaGetLastError();
 }
 

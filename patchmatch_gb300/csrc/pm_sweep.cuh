@@ -842,7 +842,15 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S
 // u8 texture 1.04 -> 0.48; 1920x960 FP16 texture 1.05 -> 0.38.  (Scoring against
 // two or four sources at a time, which then stay in L2, and combining in a second
 // kernel gains only from 5760x2880 FP16: 0.91 -> 0.73.)
-template <int S, class Img>
+// Calls of up to some 60,000 hypotheses do not fill the chip: there a row's
+// steps wait for each other, which one lane per hypothesis hid by unrolling.
+// With several sources their loads overlap; with one, the steps of a row are
+// unrolled (NT taps, known at compile time; 0: read from the arguments) so that
+// all its samples are in flight.  One source, 36 taps, kernel time with a lane
+// per hypothesis / a row step by step / unrolled: 1920x960 u8 texture, 1,000
+// hypotheses 17.5 / 21.1 / 9.2 us, 300,000 87.8 / 54.4 / 48.3; 256x128 exact,
+// 20,000 17.2 / 17.9 / 9.3, 300,000 48.0 / 55.9 / 47.2.
+template <int S, class Img, int NT>
 __global__ void __launch_bounds__(kHypThreads, 4) hyp_kernel(const __grid_constant__ HypArgs a) {
     const int own = blockIdx.x * kHypThreads + threadIdx.x;
     if ((own & ~31) >= a.n) return;
@@ -853,8 +861,8 @@ __global__ void __launch_bounds__(kHypThreads, 4) hyp_kernel(const __grid_consta
     // a warp's lanes work on each other's hypotheses: those past the end stay
     const int h = min(own, a.n - 1);
     const int2 ij = a.ij[h];
-    const int W = a.W, ph = a.patch_half, nt = ph + 1;  // 2, 4 or 6 taps a row
-    const unsigned inv = 65536u / nt + 1u;              // e / nt = e * inv >> 16 for e < 32 nt
+    const int W = a.W, ph = a.patch_half, nt = NT ? NT : ph + 1;  // 2, 4 or 6 taps a row
+    const unsigned inv = 65536u / nt + 1u;                         // e / nt = e * inv >> 16 for e < 32 nt
     const float Ic = a.ref[(size_t)ij.x * W + ij.y];
     const float px = a.planes[3 * (size_t)h], py = a.planes[3 * (size_t)h + 1], pz = a.planes[3 * (size_t)h + 2];
     const f32x2 scale = pack2(a.Wf, 2.0f * a.Hf);
@@ -863,8 +871,9 @@ __global__ void __launch_bounds__(kHypThreads, 4) hyp_kernel(const __grid_consta
     TapAccum<S, Img> acc;
     acc.zero();
     for (int k1 = -ph; k1 <= ph; k1 += 2) {
-#pragma unroll 1
-        for (int e = lane; e < 32 * nt; e += 32) {
+#pragma unroll(NT ? NT : 1)
+        for (int step = 0; step < nt; ++step) {
+            const int e = 32 * step + lane;
             const int q = (int)(e * inv >> 16), t = e - q * nt;
             const int R = __shfl_sync(~0u, ij.x, q) + k1, C = __shfl_sync(~0u, ij.y, q) + 2 * t - ph;
             const float qx = __shfl_sync(~0u, px, q), qy = __shfl_sync(~0u, py, q), qz = __shfl_sync(~0u, pz, q);
