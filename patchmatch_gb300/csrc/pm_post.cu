@@ -219,7 +219,8 @@ __global__ void clean_kernel(const __grid_constant__ CleanArgs a) {
 // All of these kernels move a few bytes per pixel; with one pixel per thread
 // they waited for their own dependent loads.  A thread takes V = 4 consecutive
 // pixels with vector accesses and keeps their gathers in flight together;
-// V = 1 where rows or maps are not aligned for that.  Measured at 3840x1920
+// V = 1 where rows or maps are not aligned for that, and for small maps (see
+// kFuseVecPixels).  Measured at 3840x1920
 // with 5 views (one pixel -> four per thread, us): init 33 -> 15, classify
 // 59/51/43/40 -> 48/42/35/31 (bound by the projection's arithmetic), resolve
 // 47/41/35/33 -> 23/17/15/14, count 21 -> 4, scan 14 -> 5, scatter 38 -> 15.
@@ -513,9 +514,18 @@ void fuse_set_poses(FuseArgs &a, int n, const double *R, const double *t) {
 }
 
 namespace {
-// Four pixels per thread where every row of every map starts on a 16-byte boundary.
+// Four pixels per thread where every row of every map starts on a 16-byte
+// boundary and the map has this many pixels.  Below, the chip holds one pixel
+// per thread in some two waves, and a thread's four projections in a row only
+// add latency.  All kernels of a fusion, one -> four pixels per thread, us:
+// 5 views 260x130 29.2 -> 37.1, 960x480 42.8 -> 48.0, 1152x576 (663,552 pixels)
+// 50.5 -> 53.3, 1216x608 (739,328) 52.6 -> 52.0, 1280x640 55.7 -> 54.8, 1920x960
+// 101 -> 92; 8 views 260x130 45.3 -> 57.5, 1152x576 71.4 -> 75.1, 1216x608 75.4 ->
+// 72.9; 2 views 260x130 14.0 -> 16.2, 1216x608 29.9 -> 30.2, 1536x768 40.0 -> 38.1.
+constexpr size_t kFuseVecPixels = 700000;
+
 bool fuse_vector(const FuseArgs &a) {
-    if (a.W % 4) return false;
+    if (a.W % 4 || (size_t)a.W * a.H < kFuseVecPixels) return false;
     uintptr_t p = (uintptr_t)a.pruned | (uintptr_t)a.target | (uintptr_t)a.depths[0];
     return (p & 15) == 0 && (((uintptr_t)a.alive | (uintptr_t)a.cls) & 3) == 0;
 }
