@@ -220,10 +220,10 @@ __global__ void clean_kernel(const __grid_constant__ CleanArgs a) {
 // they waited for their own dependent loads.  A thread takes V = 4 consecutive
 // pixels with vector accesses and keeps their gathers in flight together;
 // V = 1 where rows or maps are not aligned for that, and for small maps (see
-// kFuseVecPixels).  Measured at 3840x1920
-// with 5 views (one pixel -> four per thread, us): init 33 -> 15, classify
-// 59/51/43/40 -> 48/42/35/31 (bound by the projection's arithmetic), resolve
-// 47/41/35/33 -> 23/17/15/14, count 21 -> 4, scan 14 -> 5, scatter 38 -> 15.
+// kFuseVecPixels).  Measured at 3840x1920 with 5 views (one pixel -> four per
+// thread, us): init 33 -> 15, classify 59/51/43/40 -> 48/42/35/31 (bound by the
+// projection's arithmetic), resolve 47/41/35/33 -> 23/17/15/14, count 21 -> 4,
+// scan 14 -> 5; the scatter's figures stand at its kernel.
 enum : int8_t { kSkip = 0, kZero = 1, kDrop = 2 };
 
 template <int V, class T>
@@ -398,51 +398,48 @@ __global__ void __launch_bounds__(1024) compact_scan_kernel(unsigned *counts, in
     }
 }
 
-// Points of compaction block blockIdx.x: 256 threads with 4 pixels each.
+// Points of compaction block blockIdx.x: 256 threads, thread t with the pixels t,
+// t + 256, t + 512 and t + 768 of the block, so that the lanes of a warp read
+// and write neighbouring pixels and points.  (Four neighbouring pixels per
+// thread scatter each store over 48 bytes a lane: COUNTS.)
 __global__ void __launch_bounds__(256) compact_scatter_kernel(const __grid_constant__ FuseArgs a) {
-    __shared__ unsigned warp_tot[8];
-    const size_t N = (size_t)a.W * a.H;
-    const size_t i0 = (size_t)blockIdx.x * kCompactBlock + 4 * threadIdx.x;
+    __shared__ unsigned group_tot[32];  // kept pixels of each 32 in a row
+    const size_t N = (size_t)a.W * a.H, i0 = (size_t)blockIdx.x * kCompactBlock;
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    Vec<4, uint8_t> keep = {};
-    if (i0 + 4 <= N) {
-        keep = load_vec<4>(a.alive + i0);
-    } else {
-        for (int k = 0; k < 4; ++k)
-            if (i0 + k < N) keep.v[k] = a.alive[i0 + k];
-    }
-    const unsigned cnt = keep.v[0] + keep.v[1] + keep.v[2] + keep.v[3];
-    const unsigned inc = warp_scan(cnt);
-    if (lane == 31) warp_tot[wid] = inc;
-    __syncthreads();
-    if (!cnt) return;
-    unsigned pos = a.block_counts[blockIdx.x] + inc - cnt;
+    unsigned kept[4];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) pos += w < (int)wid ? warp_tot[w] : 0u;
-    int row = (int)(i0 / a.W), col = (int)(i0 - (size_t)row * a.W);
     for (int k = 0; k < 4; ++k) {
-        if (keep.v[k]) {
-            const size_t i = i0 + k;
-            const float d = a.depths[0][i];
-            const float2 rt = a.row_trig[row], ct = a.col_trig[col];
-            const float Xc = d * rt.x * ct.x, Yc = -d * rt.y, Zc = d * rt.x * ct.y;
-            a.xyz[3 * (size_t)pos] = a.Rinv[0] * Xc + a.Rinv[1] * Yc + a.Rinv[2] * Zc + a.tw[0];
-            a.xyz[3 * (size_t)pos + 1] = a.Rinv[3] * Xc + a.Rinv[4] * Yc + a.Rinv[5] * Zc + a.tw[1];
-            a.xyz[3 * (size_t)pos + 2] = a.Rinv[6] * Xc + a.Rinv[7] * Yc + a.Rinv[8] * Zc + a.tw[2];
-            if (a.bgr_out && a.bgr) {
-                a.bgr_out[3 * (size_t)pos] = a.bgr[3 * i];
-                a.bgr_out[3 * (size_t)pos + 1] = a.bgr[3 * i + 1];
-                a.bgr_out[3 * (size_t)pos + 2] = a.bgr[3 * i + 2];
-            }
-            if (a.ij_out) {
-                a.ij_out[2 * (size_t)pos] = row;
-                a.ij_out[2 * (size_t)pos + 1] = col;
-            }
-            ++pos;
+        const size_t i = i0 + 256 * k + threadIdx.x;
+        kept[k] = __ballot_sync(0xffffffffu, i < N && a.alive[i]);
+        if (lane == 0) group_tot[8 * k + wid] = __popc(kept[k]);
+    }
+    __syncthreads();
+    const unsigned tot = group_tot[lane];
+    const unsigned before = a.block_counts[blockIdx.x] + warp_scan(tot) - tot;  // of group `lane`
+    const size_t row0 = i0 / a.W;
+    const unsigned col0 = (unsigned)(i0 - row0 * a.W);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const unsigned first = __shfl_sync(0xffffffffu, before, 8 * k + wid);
+        if (!((kept[k] >> lane) & 1u)) continue;
+        const size_t pos = first + __popc(kept[k] & ((1u << lane) - 1u));
+        const unsigned off = 256 * k + threadIdx.x, down = (col0 + off) / (unsigned)a.W;
+        const int row = (int)(row0 + down), col = (int)(col0 + off - down * (unsigned)a.W);
+        const size_t i = i0 + off;
+        const float d = a.depths[0][i];
+        const float2 rt = a.row_trig[row], ct = a.col_trig[col];
+        const float Xc = d * rt.x * ct.x, Yc = -d * rt.y, Zc = d * rt.x * ct.y;
+        a.xyz[3 * pos] = a.Rinv[0] * Xc + a.Rinv[1] * Yc + a.Rinv[2] * Zc + a.tw[0];
+        a.xyz[3 * pos + 1] = a.Rinv[3] * Xc + a.Rinv[4] * Yc + a.Rinv[5] * Zc + a.tw[1];
+        a.xyz[3 * pos + 2] = a.Rinv[6] * Xc + a.Rinv[7] * Yc + a.Rinv[8] * Zc + a.tw[2];
+        if (a.bgr_out && a.bgr) {
+            a.bgr_out[3 * pos] = a.bgr[3 * i];
+            a.bgr_out[3 * pos + 1] = a.bgr[3 * i + 1];
+            a.bgr_out[3 * pos + 2] = a.bgr[3 * i + 2];
         }
-        if (++col == a.W) {
-            col = 0;
-            ++row;
+        if (a.ij_out) {
+            a.ij_out[2 * pos] = row;
+            a.ij_out[2 * pos + 1] = col;
         }
     }
 }
