@@ -113,15 +113,24 @@ constexpr int kMaxBands = 1024;  // counters of the banded tile order (one per S
 constexpr size_t kBandedMinRowBytes = 30000;
 constexpr size_t kBandedMinRowBytesWide = 21000;  // W >= 2880, up to 7 sources
 constexpr int kBandedWideW = 2880;
-// Images of at most this many tile rows (warps) per SM run tile_kernel_small
-// (its 16 warps per SM hold them in about one wave).  Measured against the
-// large-tile kernel, 8 sweeps, time ratio with 2 / 4 / 6 / 8 sources, textures:
-// 448x224 (10 warps per SM) 0.73 / 0.86 / 0.81 / 0.87, 512x256 (13)
-// 0.84 / 0.95 / 0.98 / 1.03, 576x288 (17) 0.93 / 0.95 / 0.92 / 0.97, 640x320
-// (21) 1.00 / 1.06 / 1.07 / 0.97.  The quad samplers, whose loads and bilinear
-// weights take more registers, gain up to 384x192 (8): 2 / 5 / 8 sources
-// 0.75 / 0.94 / 0.99, 512x256 0.95 / 1.03 / 1.02.
+// Images of at most this many tile rows (warps) per SM run tile_kernel_small:
+// an empirical line, near which the two kernels meet (16 warps per SM are
+// resident, so the largest take a little more than one wave).  Time against the
+// large-tile kernel, 8 sweeps, textures, with 2 / 4 / 6 / 7 / 8 sources:
+// 256x128 (3 warps per SM) 0.59 / 0.69 / 0.66 / 0.76 / 0.85, 384x192 (8)
+// 0.72 / 0.90 / 0.86 / 0.93 / 1.05, 448x224 (10) 0.72 / 0.80 / 0.79 / 0.82 / 0.86,
+// 512x256 (13) 0.84 / 0.96 / 0.96 / 0.97 / 1.02, 576x288 (17) 0.87 / 0.93 / 0.91 /
+// 0.99 / 0.99, 608x304 (20) 0.91 / 0.98 / 0.96 / 1.01 / 0.98, 640x320 (21) 0.96 /
+// 1.02 / 1.00 / 1.04 / 1.01.  Quad samplers: 384x192 0.77 / 0.90 / 0.90 / 0.92 /
+// 1.01, 448x224 0.74 / 0.79 / 0.78 / 0.80 / 0.83, 512x256 0.88 / 0.96 / 0.96 / 0.96 /
+// 0.99, 544x272 (16) 0.89 / 0.93 / 0.94 / 0.93 / 1.01.
 constexpr int kSmallWarpsTexture = 18, kSmallWarpsQuad = 12;
+// From this many sources on a lane gains nothing from the small kernel's extra
+// registers, and small tiles pay only where they leave the fullest SM fewer
+// rows: 8 sources, textures u8 / FP16, 320x160 (8 rows either way) 1.03 / 1.04,
+// 384x192 (8) 1.05 / 1.07, 512x256 (16) 1.02 / 1.05, but 256x128 (4 for 8)
+// 0.85 / 0.86, 448x224 (12 for 16) 0.86 / 0.87, 576x288 (20 for 24) 0.99 / 0.96.
+constexpr int kSmallBalanceSources = 8;
 // Start alignment of the per-source sampling buffers: texture objects bound
 // to pitched linear memory need the device's texture alignment (512 bytes).
 constexpr size_t kTexAlign = 512;
@@ -220,10 +229,14 @@ long long pmi::tile_warps(const pm_request *r) {
 }
 
 int pmi::tile_rows(const pm_request *r, long long warps) {
-    // all tiles resident at once: the latency of one tile visit counts
+    const long long n_sm = r->ctx->n_sm;
     const int max_warps = r->prm.sampler == PM_SAMPLER_TEXTURE ? kSmallWarpsTexture : kSmallWarpsQuad;
-    return r->S <= pm::kSmallMaxSources && warps <= (long long)max_warps * r->ctx->n_sm ? pm::kTileRowsSmall
-                                                                                       : pm::kTileRowsLarge;
+    if (r->S > pm::kSmallMaxSources || warps > max_warps * n_sm) return pm::kTileRowsLarge;
+    // rows of the fullest SM with tiles of `rows` rows
+    const auto fullest = [&](int rows) { return (warps + rows * n_sm - 1) / (rows * n_sm) * rows; };
+    if (r->S >= kSmallBalanceSources && fullest(pm::kTileRowsSmall) >= fullest(pm::kTileRowsLarge))
+        return pm::kTileRowsLarge;
+    return pm::kTileRowsSmall;
 }
 
 int pmi::tile_band(pm_request *r, dim3 grid, cudaStream_t st, pm::BandArgs *band, const pm::BandArgs **out) {
@@ -365,8 +378,12 @@ int ensure_textures(pm_request *r) {
     return PM_OK;
 }
 
-// Choose the tile height and order of a request: small tiles for images that
-// fit the chip at once (kSmallWarps*); else banded (persistent grid) for texture
+// Choose the tile height and order of a request: small tiles for small images
+// (tile_rows, from the request's own size: a served keyframe keeps that height
+// with others in flight; there, 1 / 2 / 4 in flight, 4 sweeps, small tiles take
+// 0.83 / 0.96 / 0.96 of the large ones' time at 256x128, 0.99 / 0.94 / 0.95 at
+// 320x160, 0.98 / 0.98 / 0.99 at 384x192, 0.97 / 1.02 / 1.02 at 512x256); else banded
+// (persistent grid) for texture
 // sampling when the sources' row bytes W x bytes per texel x S reach
 // kBandedMinRowBytes (kBandedMinRowBytesWide from kBandedWideW pixels wide
 // with up to 7 sources), else one CTA per tile (the quad samplers measured

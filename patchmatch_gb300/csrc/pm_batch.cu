@@ -195,8 +195,11 @@ int batch_enqueue(pm_batch *b) {
             if (b->level[x] != b->level[y]) return b->level[x] < b->level[y];
             return work(x) > work(y);
         });
-        // requests that share the device take the tile height of their sum (12
-        // requests 256 to 384 wide: 8.9 ms in large tiles, 12.0 ms in small ones)
+        // requests that share the device take the tile height of their sum: n
+        // equal ones, 4 sweeps, small against large tiles with 2 / 4 / 6 sources,
+        // 2 of 384x192 (15 warps per SM together) 0.83 / 0.92 / 0.92, 4 of 320x160
+        // (21) 0.92 / 0.98 / 1.04, 2 of 512x256 (27) 0.94 / 1.02 / 1.00, 4 of 384x192
+        // (30) 1.11 / 1.16 / 1.19, 12 of 384x192 (91) 1.21 / 1.19 / 1.22
         long long warps = 0;
         for (const pm_request *r : b->reqs) warps += pmi::tile_warps(r);
         double load[pm_batch::kBranches] = {};

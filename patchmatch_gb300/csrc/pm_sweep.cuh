@@ -736,9 +736,9 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, tile_min_blocks<S>()) t
     tile_body<S, Img, Plain, kTileH, 1, ParamAccess>(a, blockIdx.x, blockIdx.y, tile);
 }
 
-// The same visit for images whose tiles all fit the chip at once (the rule is
-// in pm_api.cu, tile_rows).  There a half-sweep lasts as long as one tile's
-// chain of costs, so the tiles have 4 rows (twice as many SMs get one), and a
+// The same visit for images of few tiles per SM (the rule is in pm_api.cu,
+// tile_rows).  There a half-sweep lasts as long as one or two tiles'
+// chains of costs, so the tiles have 4 rows (twice as many SMs get one), and a
 // lane runs the chains of several taps side by side, as many as the 128
 // registers hold that 16 warps per SM leave each thread.  Measured, 8 sweeps,
 // against the kernel above: 256x128 1 source 1.78 -> 0.95 ms, 2 sources 2.08 ->
