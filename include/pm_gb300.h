@@ -467,18 +467,21 @@ int pm_fuse_noalloc(int width, int height, int n_views, float *const *depths, co
                     uint8_t *bgr_out, int32_t *ij, unsigned *count, void *stream);
 
 /* ---- batched form ----
- * Many requests densified together: init scoring, every red/black half-sweep
- * and the post-filter run phase-major over all requests, captured once into a
- * CUDA graph and replayed by pm_batch_run.  Requests are grouped by source
- * count, image variant, propagation rule and sweep count; each phase of a
+ * Many requests densified together, captured once into a CUDA graph and
+ * replayed by pm_batch_run: init scoring, every red/black half-sweep and the
+ * post-filter.  Requests are grouped by source count, image variant,
+ * propagation rule and sweep count.  With PM_BATCH_PERSISTENT each phase of a
  * group is one persistent launch over a device queue of (request, 8x64 tile)
- * items (PM_BATCH_PERSISTENT, grid = grid_mult x resident CTAs, the groups on
- * parallel graph branches) or one launch per request (PM_BATCH_LAUNCHES); PM_BATCH_STREAMS instead runs each
- * request's whole chain on one of 8 parallel graph branches (largest request
- * first onto the least-loaded branch) so that requests overlap on the GPU;
- * PM_BATCH_MIXED is one persistent launch per phase over all requests of
- * every source count (items carry their count; the kernel holds the bodies
- * of all counts, at the register budget of the largest).  Every request's maps equal those of
+ * items (grid = grid_mult x resident CTAs).  PM_BATCH_MIXED does the same with
+ * all source counts in one group (items carry their count; the kernel holds the
+ * bodies of all counts, at the register budget of the largest), so its groups
+ * differ in image variant, propagation rule or sweep count only.  With both,
+ * the groups of a seeding level run side by side on up to 8 parallel graph
+ * branches (largest group first onto the least-loaded branch), phase by phase
+ * within a group.  PM_BATCH_LAUNCHES runs phase-major over all requests of a
+ * level, one launch per request and phase.  PM_BATCH_STREAMS runs each request's
+ * whole chain on one of the 8 branches (largest request first onto the
+ * least-loaded one).  Every request's maps equal those of
  * pm_request_run bit for bit.  Requests keep their own buffers and streams:
  * set their views before pm_batch_run; read them afterwards with
  * pm_request_read (their streams wait for the batch).  Seeded requests are
@@ -486,11 +489,12 @@ int pm_fuse_noalloc(int width, int height, int n_views, float *const *depths, co
  * the batch, or a request of the same batch, e.g. a coarse-to-fine chain whose
  * full-size request is seeded from a half-size one) are applied between the
  * init scoring and the sweeps as pm_request_run does; a request seeded from a
- * member runs one level after it (levels run in order, each level
- * phase-major), and priors from outside the batch are waited for before the
- * graph starts.  A cycle of priors within a batch is PM_EINVAL.  A request in a batch cannot be
- * destroyed (pm_request_destroy returns PM_EINVAL) until pm_batch_clear or
- * pm_batch_destroy releases it.  pm_batch_tune runs the batch once
+ * member runs one level after it (levels run in order, each finished before the
+ * next; with PM_BATCH_STREAMS on its member's branch), and priors from outside
+ * the batch are waited for before the graph starts.  A cycle of priors within a
+ * batch is PM_EINVAL, and so is a prior that has not been run with its
+ * post-filter.  A request in a batch cannot be destroyed (pm_request_destroy
+ * returns PM_EINVAL) until pm_batch_clear or pm_batch_destroy releases it.  pm_batch_tune runs the batch once
  * per executor candidate, keeps the fastest and reports the timings.
  * No counterpart in the reference (one keyframe at a time,
  * depthmap_computation_module.cc:205-472). */

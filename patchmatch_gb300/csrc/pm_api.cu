@@ -382,12 +382,11 @@ int ensure_textures(pm_request *r) {
 // (tile_rows, from the request's own size: a served keyframe keeps that height
 // with others in flight; there, 1 / 2 / 4 in flight, 4 sweeps, small tiles take
 // 0.83 / 0.96 / 0.96 of the large ones' time at 256x128, 0.99 / 0.94 / 0.95 at
-// 320x160, 0.98 / 0.98 / 0.99 at 384x192, 0.97 / 1.02 / 1.02 at 512x256); else banded
-// (persistent grid) for texture
-// sampling when the sources' row bytes W x bytes per texel x S reach
-// kBandedMinRowBytes (kBandedMinRowBytesWide from kBandedWideW pixels wide
-// with up to 7 sources), else one CTA per tile (the quad samplers measured
-// 4-6 % slower banded at 1920x960).
+// 320x160, 0.98 / 0.98 / 0.99 at 384x192, 0.97 / 1.02 / 1.02 at 512x256); else
+// banded (persistent grid) for texture sampling when the sources' row bytes
+// W x bytes per texel x S reach kBandedMinRowBytes (kBandedMinRowBytesWide from
+// kBandedWideW pixels wide with up to 7 sources), else one CTA per tile (the quad
+// samplers measured 4-6 % slower banded at 1920x960).
 void set_tile_order(pm_request *r) {
     r->banded_blocks = 0;
     r->tile_rows = pmi::tile_rows(r, pmi::tile_warps(r));

@@ -17,14 +17,15 @@ using pmi::fail;
 using pmi::fill_args;
 
 // ---------------------------------------------------------------------------
-// Batched executor: many requests densified by phase-major launches (init
-// scoring, then each red/black half-sweep of every request, then the
-// post-filter), captured once into a CUDA graph and replayed.  Requests are
-// grouped by (source count, image variant, propagation rule, sweep count);
-// each phase of a group is one persistent launch over a device queue of
-// (request, tile) items (PM_BATCH_PERSISTENT; the groups on parallel graph
-// branches) or one launch per request (PM_BATCH_LAUNCHES).  A tile's update reads only pixels of the other colour,
-// so the result of every request is the same as from pm_request_run.
+// Batched executor: many requests densified together (init scoring, each
+// red/black half-sweep, post-filter), captured once into a CUDA graph and
+// replayed.  Requests are grouped by (source count, image variant, propagation
+// rule, sweep count), PM_BATCH_MIXED by all but the source count; each phase of a
+// group is one persistent launch over a device queue of (request, tile) items
+// (PM_BATCH_PERSISTENT, PM_BATCH_MIXED; the groups of a level on parallel graph
+// branches) or one launch per request (PM_BATCH_LAUNCHES).  PM_BATCH_STREAMS has
+// whole requests on the branches.  A tile's update reads only pixels of the other
+// colour, so the result of every request is the same as from pm_request_run.
 // ---------------------------------------------------------------------------
 struct pm_batch {
     struct Group {
@@ -45,7 +46,7 @@ struct pm_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     std::vector<cudaEvent_t> req_events;
-    static constexpr int kBranches = 8;      // PM_BATCH_STREAMS: parallel chains of requests
+    static constexpr int kBranches = 8;      // parallel graph branches (of groups or, PM_BATCH_STREAMS, of requests)
     cudaStream_t branch[kBranches] = {};
     cudaEvent_t fork = nullptr, join[kBranches] = {};
     cudaGraph_t graph = nullptr;

@@ -85,10 +85,11 @@ cudaError_t configure_batch_mixed<PM_MIXED_KIND>() {
 template <>
 int batch_mixed_blocks_per_sm<PM_MIXED_KIND>(bool plain) {
     int n = 0;
+    constexpr int threads = Geo<kTileH>::kThreads;
     if (plain)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<true>, Geo<kTileH>::kThreads, tile_kernel_smem_max());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<true>, threads, tile_kernel_smem_max());
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<false>, Geo<kTileH>::kThreads, tile_kernel_smem_max());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_kernel<false>, threads, tile_kernel_smem_max());
     return n;
 }
 

@@ -492,7 +492,9 @@ struct TapAccum {
         const float sbx = flip_sign(bx, sg), sby = flip_sign(by, sg), sbz = flip_sign(bz, sg);
         const f32x2 bx2 = pack2(sbx, sbx), by2 = pack2(sby, sby), bz2 = pack2(sbz, sbz);
         add_rot(P, src, scale, half, shift, fabsf(s),
-                [&](int r) { return rotate(Acc::row(P.G[r][0]), Acc::row(P.G[r][1]), Acc::row(P.G[r][2]), bx2, by2, bz2); },
+                [&](int r) {
+                    return rotate(Acc::row(P.G[r][0]), Acc::row(P.G[r][1]), Acc::row(P.G[r][2]), bx2, by2, bz2);
+                },
                 w, xs);
     }
     // The footprints of the tap at the grid point with row trig rt = (cos lat,

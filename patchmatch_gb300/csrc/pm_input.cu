@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(kVecThreads)
     uint32_t a[4 * CH], b[4 * CH];
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(r0) + c), w = __ldg(reinterpret_cast<const uint4 *>(r1) + c);
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(r0) + c);
+        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(r1) + c);
         a[4 * c] = v.x; a[4 * c + 1] = v.y; a[4 * c + 2] = v.z; a[4 * c + 3] = v.w;
         b[4 * c] = w.x; b[4 * c + 1] = w.y; b[4 * c + 2] = w.z; b[4 * c + 3] = w.w;
     }
@@ -214,7 +215,10 @@ __global__ void __launch_bounds__(kVecThreads)
 }
 
 // Blocks of kVecThreads threads for n items of `per` each along a row.
-unsigned vec_blocks(size_t n, int per) { return (unsigned)((n + (size_t)kVecThreads * per - 1) / ((size_t)kVecThreads * per)); }
+unsigned vec_blocks(size_t n, int per) {
+    const size_t items = (size_t)kVecThreads * per;
+    return (unsigned)((n + items - 1) / items);
+}
 
 constexpr int kMaxGridY = 65535;  // rows of a launch with one row per blockIdx.y
 
@@ -260,8 +264,8 @@ int pm_image_resize(pm_ctx *ctx, const void *src, int sw, int sh, size_t spitch,
     const uint8_t *s = (const uint8_t *)src;
     uint8_t *d = (uint8_t *)dst;
     // (2 x + 1/2 is exact in FP32 up to 2^22 outputs)
-    if (sw == 2 * (int64_t)dw && sh == 2 * (int64_t)dh && dw <= (1 << 21) && aligned16(s, spitch) && (((uintptr_t)d | dpitch) & 7) == 0 &&
-        dh <= kMaxGridY) {
+    if (sw == 2 * (int64_t)dw && sh == 2 * (int64_t)dh && dw <= (1 << 21) && aligned16(s, spitch) &&
+        (((uintptr_t)d | dpitch) & 7) == 0 && dh <= kMaxGridY) {
         const dim3 grid(vec_blocks(dw, 8), dh);
         switch (channels) {
             case 1: halve_vec_kernel<1><<<grid, kVecThreads, 0, st>>>(s, spitch, d, dw, dpitch); break;
@@ -289,7 +293,8 @@ int pm_build_pyramid_f16(pm_ctx *ctx, const void *src, int W, int H, size_t pitc
         const bool packed = pitch == (size_t)W;
         const size_t n = packed ? (size_t)W * H : (size_t)W;
         const int rows = packed ? 1 : H;
-        if (aligned16(src, rows > 1 ? pitch : 0) && aligned16(out[0], rows > 1 ? (size_t)W * 2 : 0) && rows <= kMaxGridY)
+        if (aligned16(src, rows > 1 ? pitch : 0) && aligned16(out[0], rows > 1 ? (size_t)W * 2 : 0) &&
+            rows <= kMaxGridY)
             u8_to_half_vec_kernel<<<dim3(vec_blocks(n, 16), rows), kVecThreads, 0, st>>>((const uint8_t *)src, n, pitch,
                                                                                          (__half *)out[0], W);
         else

@@ -41,9 +41,10 @@ constexpr int kNbr = 8;
 // staged tile, the parked state, the scratch of the speculative propagation
 // pass (see tile_body: reference moments per pixel, candidate scores and best
 // sources per (candidate, pixel), the (pixel, candidate) work list, outcome bits
-// per pixel, per-warp scan totals) and the warp factors (per source: A of both column parities, B
-// of both signs); the rest of the SM's unified L1/shared storage stays L1 for
-// the texture samples, whose hit rate sets the kernel's speed.
+// per pixel, per-warp scan totals) and the warp factors (per source: A of both
+// column parities, B of both signs); the rest of the SM's unified L1/shared
+// storage stays L1 for the texture samples, whose hit rate sets the kernel's
+// speed.
 constexpr int kFactorA = 2 * kTileCols;  // (column parity, same-colour column)
 template <int TH>
 struct Geo {
@@ -158,7 +159,8 @@ struct Park {
     static constexpr unsigned kStride = 4u * Geo<TH>::kThreads;
     unsigned base;
     __device__ __forceinline__ explicit Park(const unsigned char *smem)
-        : base((unsigned)__cvta_generic_to_shared(reinterpret_cast<const float *>(smem + Geo<TH>::kPark) + threadIdx.x)) {}
+        : base((unsigned)__cvta_generic_to_shared(reinterpret_cast<const float *>(smem + Geo<TH>::kPark) +
+                                                  threadIdx.x)) {}
     __device__ __forceinline__ void put(int k, float v) const {
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + kStride * k), "f"(v) : "memory");
     }
@@ -404,8 +406,8 @@ __device__ __forceinline__ void spec_round(const A &a, const float4 *tile, const
 // Measured, 8 sweeps, both together: 1920x960, 6 sources 58.0 -> 53.4 ms;
 // 512x256, 4 sources 5.06 -> 4.4 ms.  The host variant (Plain) needs one round
 // only, since its costs do not depend on the state, and skips every candidate
-// that did not change: 5 exact sources,
-// 641x321 12.0 -> 9.9 ms, 512x256 8.4 -> 6.6 ms.
+// that did not change: 5 exact sources, 641x321 12.0 -> 9.9 ms, 512x256 8.4 ->
+// 6.6 ms.
 template <int S, class Img, bool Plain, int TH, int U, class Acc, class A>
 __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *tile) {
     using G = Geo<TH>;
@@ -465,7 +467,7 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
     float hx = cur.x, hy = cur.y, hz = cur.z;   // plane_*_hyp of the reference
     float curr_depth = cur.w;
     float cand_w = cand.w;
-    bool moved = false;    // a plane was taken (plain propagation: a neighbour's)
+    bool moved = false;    // a plane was taken (until the refinements: a neighbour's)
     int h = 0;
 
     if (spec) {
@@ -478,7 +480,8 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
         const int8_t *res_best = reinterpret_cast<const int8_t *>(smem + G::kBest);
         unsigned *flag = reinterpret_cast<unsigned *>(smem + G::kFlag) + tid;
         const auto nbr_plane = [&](int n) {
-            return n < kNbr && nbr_inside(n, i, j, W, H) ? a.plane[nbr_index(n, i, j, W)] : make_float4(0.f, 0.f, 0.f, 0.f);
+            return n < kNbr && nbr_inside(n, i, j, W, H) ? a.plane[nbr_index(n, i, j, W)]
+                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         // Candidates that can be accepted in the state before propagation.  A
         // propagated plane is scored as NCC x f with a smoothness factor f in
@@ -731,16 +734,17 @@ __device__ __forceinline__ void tile_body(const A &a, int bx, int by, float4 *ti
 }
 
 template <int S, class Img, bool Plain>
-__global__ void __launch_bounds__(Geo<kTileH>::kThreads, tile_min_blocks<S>()) tile_kernel(const __grid_constant__ SweepArgs a) {
+__global__ void __launch_bounds__(Geo<kTileH>::kThreads, tile_min_blocks<S>())
+    tile_kernel(const __grid_constant__ SweepArgs a) {
     extern __shared__ float4 tile[];
     tile_body<S, Img, Plain, kTileH, 1, ParamAccess>(a, blockIdx.x, blockIdx.y, tile);
 }
 
 // The same visit for images of few tiles per SM (the rule is in pm_api.cu,
-// tile_rows).  There a half-sweep lasts as long as one or two tiles'
-// chains of costs, so the tiles have 4 rows (twice as many SMs get one), and a
-// lane runs the chains of several taps side by side, as many as the 128
-// registers hold that 16 warps per SM leave each thread.  Measured, 8 sweeps,
+// tile_rows).  There a half-sweep lasts as long as one or two tiles' chains of
+// costs, so the tiles have 4 rows (twice as many SMs get one), and a lane runs
+// the chains of several taps side by side, as many as the 128 registers hold that
+// 16 warps per SM leave each thread.  Measured, 8 sweeps,
 // against the kernel above: 256x128 1 source 1.78 -> 0.95 ms, 2 sources 2.08 ->
 // 1.25 ms, 4 sources 3.34 -> 2.00 ms; 512x256 2 sources 3.05 -> 2.51 ms, 4
 // sources 4.48 -> 4.15 ms.  Taps at once at 256x128, 2 / 3 / 6: 1 source 1.25 /
@@ -803,7 +807,8 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S
 // other (a half-sweep reads only the other colour), so no CTA waits on
 // another; phases are separated by kernel boundaries.
 template <int S, class Img, bool Plain>
-__global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S>()) batch_kernel(const __grid_constant__ BatchArgs b) {
+__global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S>())
+    batch_kernel(const __grid_constant__ BatchArgs b) {
     extern __shared__ float4 tile[];
     __shared__ SweepArgs sa;
     __shared__ int s_item;
