@@ -847,6 +847,11 @@ __global__ void __launch_bounds__(Geo<kTileH>::kThreads, persistent_min_blocks<S
 // u8 texture 1.04 -> 0.48; 1920x960 FP16 texture 1.05 -> 0.38.  (Scoring against
 // two or four sources at a time, which then stay in L2, and combining in a second
 // kernel gains only from 5760x2880 FP16: 0.91 -> 0.73.)
+// Hypotheses of neighbouring pixels in raster order, whose lanes share sectors
+// anyway, pay for the exchange: 300,000 at 1920x960, u8 texture with 2 sources
+// 58 -> 67 us and with 8 193 -> 191, FP16 footprints with 4 sources 126 -> 138, 1 to
+// 3 % of the call.  (A branch that left such warps one lane per hypothesis gave
+// back half of that.)
 // Calls of up to some 60,000 hypotheses do not fill the chip: there a row's
 // steps wait for each other, which one lane per hypothesis hid by unrolling.
 // With several sources their loads overlap; with one, the steps of a row are
