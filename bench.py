@@ -81,13 +81,15 @@ def _mpix_views(ms: float) -> float:
 
 
 def _samples_per_half_sweep() -> float:
+    """Nominal samples of one half-sweep: every pixel's 14 candidates, as the
+    reference scores them.  The kernel skips those that cannot be accepted."""
     ph = 5
     interior = (W - 2 * (ph + 1) + 1) * (H - 2 * (ph + 1) + 1)
     return interior / 2 * 14 * S * 36
 
 
 def _samples_per_step() -> float:
-    """Algorithmic samples of one keyframe's densification: init scoring (one
+    """Nominal samples of one keyframe's densification: init scoring (one
     hypothesis per interior pixel) and 2 x SWEEPS half-sweeps of 14."""
     return _samples_per_half_sweep() * (2 * SWEEPS + 1 / 7)
 
@@ -184,12 +186,15 @@ def _hbm_view(traffic, launch_ms):
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)"}
 
 
-# DRAM bytes of one sweep launch of this workload, from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum), valid only for the kernel
-# sources it was measured on: a different build reports null rather than a
-# stale figure.
-TRAFFIC_NCU = {"bytes_per_launch": 59997440,
-               "sources_sha256": "2b55b01ae79f6076398ee3301797989196a91dcf356a5742ec497b02b092f42d"}
+# Counters of this workload's launches from ncu captures (--profile-sweep),
+# valid only for the kernel sources they were taken on: a different build
+# reports null rather than a stale figure.  DRAM bytes of the 8th half-sweep
+# (dram__bytes_read.sum + dram__bytes_write.sum); samples that were scored:
+# texture instructions x active lanes (smsp__inst_executed_op_texture.sum x
+# smsp__thread_inst_executed_per_inst_executed.ratio), summed over the 16
+# half-sweeps, and over those and the two launches of the init scoring.
+NCU = {"bytes_per_launch": 60010496, "sweep_samples": 25129033853, "step_samples": 25517314546,
+       "sources_sha256": "91e84aaed48dd0584f5fe820d6caf3a90ec3caa6dee748b41b72585ebd83eb6c"}
 KERNEL_SOURCES = ("patchmatch_gb300/csrc/pm_sweep.cuh", "patchmatch_gb300/csrc/pm_device.cuh",
                   "patchmatch_gb300/csrc/pm_inst.cu", "patchmatch_gb300/csrc/pm_types.h")
 
@@ -203,10 +208,8 @@ def kernel_sources_sha256() -> str:
     return h.hexdigest()
 
 
-def _traffic():
-    if TRAFFIC_NCU["bytes_per_launch"] is None or TRAFFIC_NCU["sources_sha256"] != kernel_sources_sha256():
-        return None
-    return TRAFFIC_NCU["bytes_per_launch"]
+def _counted(key):
+    return NCU[key] if NCU["sources_sha256"] == kernel_sources_sha256() else None
 
 
 def cpu_sample(target_s: float = 12.0, threads: int = 0):
@@ -854,8 +857,9 @@ def run_ours(args):
     fused_points = int(ks.count.item())
     cleaned_valid = float((ks.cleaned > 0).float().mean().item())
 
-    # --- dominant kernel: one red-black half-sweep, timed on the request's stream ---
+    # --- dominant kernel: one red-black half-sweep, the mean of a keyframe's 16 on the request's stream ---
     r.run()
+    r.init()
     nhalf = 2 * SWEEPS
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     with torch.cuda.stream(stream):
@@ -865,7 +869,6 @@ def run_ours(args):
         e1.record(stream)
     r.synchronize()
     sweep_ms = e0.elapsed_time(e1) / nhalf
-    achieved = FLOP_PER_SAMPLE * _samples_per_half_sweep() / (sweep_ms * 1e-3) / 1e12
     peak = ctx.probe_fp32_peak()
 
     # --- end to end through the C ABI from pinned host buffers ---
@@ -946,14 +949,17 @@ def run_ours(args):
     batched = None if args.no_batched else _optional(run_batched, native, scene, ctx, local, args)
     precision = None if args.no_precision else _optional(run_precision, native, scene, ctx, local)
     pipeline = _optional(run_pipeline, native, scene, ctx, local, args.steps)
-    traffic = _traffic()
+    traffic = _counted("bytes_per_launch")
     # the roofline terms of the cost kernel (samples/s): 40 FP32 flop, 4
     # special-function operations and 1 bilinear fetch per sample
     sfu = ctx.probe_sfu_peak()
     tex = ctx.probe_tex_peak()
     terms = {"fp32": peak * 1e12 / FLOP_PER_SAMPLE, "sfu": sfu * 1e9 / SFU_PER_SAMPLE, "tex": tex * 1e9}
     binding = min(terms, key=terms.get)
-    samples_s = _samples_per_half_sweep() / (sweep_ms * 1e-3)
+    scored, scored_step = _counted("sweep_samples"), _counted("step_samples")
+    samples_s = scored / nhalf / (sweep_ms * 1e-3) if scored else None
+    achieved = FLOP_PER_SAMPLE * samples_s / 1e12 if scored else None
+    nominal_s = _samples_per_half_sweep() / (sweep_ms * 1e-3)
     line = None
     if rank == 0:
         cpu = None
@@ -983,21 +989,30 @@ def run_ours(args):
                             "pm_filter_consistency_device, pm_fuse_device -> cleaned depth, score and fused "
                             "points (xyz, pixel) to pinned host memory"},
             "roofline": {"bound": "fp32", "kernel": "tile_kernel (red-black half-sweep)",
-                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
+                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                         "frac": achieved / peak if scored else None,
                          "peak_source": "in-run FFMA probe (pm_probe_fp32_peak); MEASURED_PEAKS.json has no FP32 figure",
-                         "flop_per_sample": FLOP_PER_SAMPLE, "samples_per_launch": _samples_per_half_sweep(),
+                         "flop_per_sample": FLOP_PER_SAMPLE, "samples_per_launch": scored / nhalf if scored else None,
+                         "samples_source": "samples that were scored (ncu, current sources, mean of the keyframe's "
+                                           "half-sweeps), null when the kernel sources differ from the profiled",
                          "launch_ms": sweep_ms, "traffic": traffic,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the current sources' "
                                            "sweep kernel, null when the kernel sources differ from the profiled",
                          "terms_samples_per_s": terms, "binding_term": binding,
-                         "achieved_samples_per_s": samples_s, "frac_of_binding": samples_s / terms[binding],
+                         "achieved_samples_per_s": samples_s,
+                         "frac_of_binding": samples_s / terms[binding] if scored else None,
+                         "nominal_equivalent": {
+                             "samples_per_launch": _samples_per_half_sweep(), "samples_per_s": nominal_s,
+                             "tflops": FLOP_PER_SAMPLE * nominal_s / 1e12,
+                             "note": "as if all 14 candidates of every pixel were scored; not a rate of the hardware"},
                          "probes": {"fp32_tflops": peak, "sfu_gops": sfu, "tex_gfetches": tex},
                          "hbm_view": _hbm_view(traffic, sweep_ms)},
             "value_vs_roofline": {
-                "samples_per_step": _samples_per_step(),
-                "frac": {k: _samples_per_step() / v / (ms_step / 1e3) for k, v in terms.items()},
+                "samples_per_step": scored_step,
+                "frac": {k: scored_step / v / (ms_step / 1e3) for k, v in terms.items()} if scored_step else None,
+                "nominal_samples_per_step": _samples_per_step(),
                 "note": "the whole step (densification, post-filter, consistency filter, fusion) against the "
-                        "time its algorithmic samples take at each roofline term"},
+                        "time that the samples it scores take at each roofline term"},
             "served": served,
             "batched": batched,
             "precision": precision,
@@ -1025,8 +1040,8 @@ def run_ours(args):
 def run_profile_sweep():
     """One densification of the 1920x960x6 keyframe (init scoring, 16
     half-sweeps, post-filter) and nothing else: the case the sweep kernel's
-    ncu captures select launches from (tile_kernel launch 0 is the init
-    scoring, launch k the k-th half-sweep)."""
+    ncu captures select launches from (tile_kernel launches 0 and 1 are the
+    init scoring, launch k + 1 the k-th half-sweep)."""
     from patchmatch_gb300 import native, scene
     req = scene.config_request(2, seed=0)
     with native.Context(0) as ctx:
