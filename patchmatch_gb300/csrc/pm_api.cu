@@ -131,6 +131,13 @@ constexpr int kSmallWarpsTexture = 18, kSmallWarpsQuad = 12;
 // 384x192 (8) 1.05 / 1.07, 512x256 (16) 1.02 / 1.05, but 256x128 (4 for 8)
 // 0.85 / 0.86, 448x224 (12 for 16) 0.86 / 0.87, 576x288 (20 for 24) 0.99 / 0.96.
 constexpr int kSmallBalanceSources = 8;
+// Tile rows per SM of the other requests in flight from which a small image runs
+// in large tiles too: n equal requests in flight, 8 sweeps, all in small against
+// all in large tiles, textures, 2 / 4 / 6 / 8 sources (warps per SM of the others):
+// 2 of 512x256 (13) 0.92 / 1.00 / 0.98 / 1.00, 3 of 384x192 (15) 0.91 / 0.97 / 0.98 /
+// 1.06, 2 of 576x288 (17) 1.05 / 1.11 / 1.10 / 1.01, 3 of 448x224 (21) 1.09 / 1.15 /
+// 1.13 / 1.05, 8 of 256x128 (24) 1.06 / 1.11 / 1.32 / 1.48.
+constexpr int kSharedWarps = 16;
 // Start alignment of the per-source sampling buffers: texture objects bound
 // to pitched linear memory need the device's texture alignment (512 bytes).
 constexpr size_t kTexAlign = 512;
@@ -228,10 +235,15 @@ long long pmi::tile_warps(const pm_request *r) {
     return (long long)((r->W + pm::kTileWidth - 1) / pm::kTileWidth) * r->H;
 }
 
+// Whether `warps` tile rows of the request's kind are few enough for small tiles.
+static bool few_tile_rows(const pm_request *r, long long warps) {
+    const int max_warps = r->prm.sampler == PM_SAMPLER_TEXTURE ? kSmallWarpsTexture : kSmallWarpsQuad;
+    return r->S <= pm::kSmallMaxSources && warps <= (long long)max_warps * r->ctx->n_sm;
+}
+
 int pmi::tile_rows(const pm_request *r, long long warps) {
     const long long n_sm = r->ctx->n_sm;
-    const int max_warps = r->prm.sampler == PM_SAMPLER_TEXTURE ? kSmallWarpsTexture : kSmallWarpsQuad;
-    if (r->S > pm::kSmallMaxSources || warps > max_warps * n_sm) return pm::kTileRowsLarge;
+    if (!few_tile_rows(r, warps)) return pm::kTileRowsLarge;
     // rows of the fullest SM with tiles of `rows` rows
     const auto fullest = [&](int rows) { return (warps + rows * n_sm - 1) / (rows * n_sm) * rows; };
     if (r->S >= kSmallBalanceSources && fullest(pm::kTileRowsSmall) >= fullest(pm::kTileRowsLarge))
@@ -239,9 +251,70 @@ int pmi::tile_rows(const pm_request *r, long long warps) {
     return pm::kTileRowsSmall;
 }
 
-int pmi::tile_band(pm_request *r, dim3 grid, cudaStream_t st, pm::BandArgs *band, const pm::BandArgs **out) {
+void pmi::note_running(pm_request *r) {
+    std::vector<pm_request *> &v = r->ctx->running;
+    if (std::find(v.begin(), v.end(), r) == v.end()) v.push_back(r);
+}
+
+// What the request's stream is doing; waiting: for a prior that is unfinished.
+enum class StreamState { done, waiting, working };
+static StreamState stream_state(const pm_request *q) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(q->stream, &cap) != cudaSuccess) return StreamState::done;
+    if (cap != cudaStreamCaptureStatusNone) return StreamState::working;
+    if (cudaStreamQuery(q->stream) != cudaErrorNotReady) return StreamState::done;
+    const cudaEvent_t prior = q->prior_res ? q->prior_res->ready : q->prior ? q->prior->ready : nullptr;
+    return prior && cudaEventQuery(prior) == cudaErrorNotReady ? StreamState::waiting : StreamState::working;
+}
+
+// Choose the tile height of the request's next launches: large tiles when the
+// other requests of the context at work have kSharedWarps tile rows per SM, else
+// by its own size.  They are those on the device now or, if more, those that
+// joined it during its last run: the first of a burst is alone when it is
+// enqueued.  1 / 2 / 4 / 8 / 12 requests of 384x192 with 4 sources in flight, 8
+// sweeps, every height by the request's own size: 2.55 / 3.52 / 6.62 / 13.3 / 19.8 ms,
+// by this rule 2.55 / 3.51 / 5.73 / 11.2 / 16.7.
+static void choose_tile_rows(pm_request *r) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(r->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+    const long long own = pmi::tile_warps(r), shared = (long long)kSharedWarps * r->ctx->n_sm;
+    std::vector<pm_request *> &run = r->ctx->running;
+    std::vector<pm_request *> busy;
+    long long others = 0;
+    // the queries must not break a capture that the caller has open on this thread
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    size_t kept = 0;
+    for (pm_request *q : run) {
+        if (q == r) continue;
+        if (others < shared || q->company < shared) {  // else the answer changes nothing
+            const StreamState state = stream_state(q);
+            if (state == StreamState::done) continue;
+            if (state == StreamState::working) {
+                others += pmi::tile_warps(q);
+                busy.push_back(q);
+            }
+        }
+        run[kept++] = q;
+    }
+    run.resize(kept);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // the answer of a query, not an error
+    for (pm_request *q : busy) q->company = std::max(q->company, others + own - pmi::tile_warps(q));
+    const long long company = std::max(others, r->company);
+    // the balance rule of tile_rows was measured on whole runs of one request
+    if (company == 0 && !r->prior && !r->prior_res)
+        r->tile_rows = pmi::tile_rows(r, own);
+    else
+        r->tile_rows = company < shared && few_tile_rows(r, own) ? pm::kTileRowsSmall : pm::kTileRowsLarge;
+    r->company = others;
+    pmi::note_running(r);
+}
+
+int pmi::tile_band(pm_request *r, int rows, dim3 grid, cudaStream_t st, pm::BandArgs *band,
+                   const pm::BandArgs **out) {
     *out = nullptr;
-    if (r->banded_blocks <= 0) return PM_OK;
+    if (rows != pm::kTileRowsLarge || r->banded_blocks <= 0) return PM_OK;
     const int n_sm = r->ctx->n_sm, segs = (n_sm + (int)grid.x - 1) / (int)grid.x;
     band->ctr = r->band_ctr;
     band->tiles_x = (int)grid.x;
@@ -378,19 +451,14 @@ int ensure_textures(pm_request *r) {
     return PM_OK;
 }
 
-// Choose the tile height and order of a request: small tiles for small images
-// (tile_rows, from the request's own size: a served keyframe keeps that height
-// with others in flight; there, 1 / 2 / 4 in flight, 4 sweeps, small tiles take
-// 0.83 / 0.96 / 0.96 of the large ones' time at 256x128, 0.99 / 0.94 / 0.95 at
-// 320x160, 0.98 / 0.98 / 0.99 at 384x192, 0.97 / 1.02 / 1.02 at 512x256); else
-// banded (persistent grid) for texture sampling when the sources' row bytes
-// W x bytes per texel x S reach kBandedMinRowBytes (kBandedMinRowBytesWide from
-// kBandedWideW pixels wide with up to 7 sources), else one CTA per tile (the quad
-// samplers measured 4-6 % slower banded at 1920x960).
+// Choose the tile order of a request's large tiles: banded (persistent grid) for
+// texture sampling when the sources' row bytes W x bytes per texel x S reach
+// kBandedMinRowBytes (kBandedMinRowBytesWide from kBandedWideW pixels wide with
+// up to 7 sources), else one CTA per tile (the quad samplers measured 4-6 %
+// slower banded at 1920x960).
 void set_tile_order(pm_request *r) {
     r->banded_blocks = 0;
     r->tile_rows = pmi::tile_rows(r, pmi::tile_warps(r));
-    if (r->tile_rows == pm::kTileRowsSmall) return;
     if (r->ctx->n_sm <= 0 || r->ctx->n_sm > kMaxBands / 2 || r->prm.sampler != PM_SAMPLER_TEXTURE) return;
     const size_t texel = r->prm.image_format == PM_IMAGE_F16 ? 2 : 1;
     const size_t min_row = (r->W >= kBandedWideW && r->S <= 7) ? kBandedMinRowBytesWide : kBandedMinRowBytes;
@@ -410,7 +478,7 @@ int launch_tile(pm_request *r, int mode, int colour, int sweep, cudaStream_t st 
     const dim3 grid = pm::tile_grid(r->W, r->H, r->tile_rows);
     pm::BandArgs band{};
     const pm::BandArgs *bp = nullptr;
-    const int rc = pmi::tile_band(r, grid, st, &band, &bp);
+    const int rc = pmi::tile_band(r, r->tile_rows, grid, st, &band, &bp);
     if (rc) return rc;
     cudaError_t e = pm::dispatch_tile(r->S, kind, r->tile_rows, grid, st, a, bp);
     r->ctx->launches++;
@@ -1049,8 +1117,11 @@ int pm_request_destroy(pm_request *r) {
     unlink_dependents(r->dependents, true);
     link_prior(r, nullptr, nullptr);
     cudaStreamSynchronize(r->stream);
-    if (r->gexec) cudaGraphExecDestroy(r->gexec);
-    if (r->graph) cudaGraphDestroy(r->graph);
+    for (const pm_request::RunGraph *g : {&r->small_run, &r->large_run}) {
+        if (g->exec) cudaGraphExecDestroy(g->exec);
+        if (g->graph) cudaGraphDestroy(g->graph);
+    }
+    ctx->running.erase(std::remove(ctx->running.begin(), ctx->running.end(), r), ctx->running.end());
     destroy_textures(r);
     if (r->lm) cudaFree(r->lm);
     cudaEventDestroy(r->ready);
@@ -1126,6 +1197,7 @@ int pm_request_init(pm_request *r) {
     PM_CUDA(r->ctx, cudaSetDevice(r->ctx->device));
     fill_args(r);
     r->postprocessed = false;
+    choose_tile_rows(r);
     return enqueue_init(r);
 }
 
@@ -1163,6 +1235,7 @@ int pm_request_sweep(pm_request *r, int first_half, int n_half) {
     PM_CUDA(r->ctx, cudaSetDevice(r->ctx->device));
     fill_args(r);
     r->postprocessed = false;
+    choose_tile_rows(r);
     return enqueue_sweeps(r, first_half, n_half);
 }
 
@@ -1302,7 +1375,11 @@ int pm_request_run(pm_request *r) {
     int rc = check_views(r);
     if (rc) return rc;
     PM_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (r->graph_dirty || !r->gexec) {
+    choose_tile_rows(r);
+    if (r->graph_dirty) r->small_run.current = r->large_run.current = false;
+    r->graph_dirty = false;
+    pm_request::RunGraph &run = r->tile_rows == pm::kTileRowsSmall ? r->small_run : r->large_run;
+    if (!run.current) {
         NvtxRange capture("capture sweep graph");
         fill_args(r);
         cudaGraph_t g = nullptr;
@@ -1317,24 +1394,24 @@ int pm_request_run(pm_request *r) {
         if (ce != cudaSuccess) return fail(ctx, PM_ECUDA, "graph capture: %s", cudaGetErrorString(ce));
         ctx->launches = before;  // counted again on replay below
         bool updated = false;
-        if (r->gexec) {
+        if (run.exec) {
             cudaGraphExecUpdateResultInfo info;
-            if (cudaGraphExecUpdate(r->gexec, g, &info) == cudaSuccess) updated = true;
+            if (cudaGraphExecUpdate(run.exec, g, &info) == cudaSuccess) updated = true;
             else cudaGetLastError();
         }
         if (!updated) {
-            if (r->gexec) cudaGraphExecDestroy(r->gexec);
-            r->gexec = nullptr;
-            PM_CUDA(ctx, cudaGraphInstantiate(&r->gexec, g, 0));
+            if (run.exec) cudaGraphExecDestroy(run.exec);
+            run.exec = nullptr;
+            PM_CUDA(ctx, cudaGraphInstantiate(&run.exec, g, 0));
         }
-        if (r->graph) cudaGraphDestroy(r->graph);
-        r->graph = g;
-        r->graph_dirty = false;
+        if (run.graph) cudaGraphDestroy(run.graph);
+        run.graph = g;
+        run.current = true;
     }
     rc = wait_for_prior(r, r->prior);
     if (rc) return rc;
     if (r->prior_res) PM_CUDA(ctx, cudaStreamWaitEvent(r->stream, r->prior_res->ready, 0));
-    PM_CUDA(ctx, cudaGraphLaunch(r->gexec, r->stream));
+    PM_CUDA(ctx, cudaGraphLaunch(run.exec, r->stream));
     ctx->launches += 3 + 2 * (uint64_t)r->prm.iterations + (r->prm.postprocess ? 3 : 0) +
                      ((r->prior || r->prior_res) ? 4 : 0) + (r->n_lm > 0 ? 3 : 0);
     r->postprocessed = r->prm.postprocess != 0;

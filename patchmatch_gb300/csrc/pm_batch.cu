@@ -227,7 +227,7 @@ int batch_enqueue(pm_batch *b) {
                 const dim3 grid = pm::tile_grid(r->W, r->H, rows);
                 pm::BandArgs band{};
                 const pm::BandArgs *bp = nullptr;
-                const int rc = pmi::tile_band(r, grid, bs, &band, &bp);
+                const int rc = pmi::tile_band(r, rows, grid, bs, &band, &bp);
                 if (rc) return rc;
                 cudaError_t e = pm::dispatch_tile(r->S, kind, rows, grid, bs, a, bp);
                 if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
@@ -296,11 +296,11 @@ int batch_enqueue(pm_batch *b) {
             a.colour = colour;
             a.sweep = sweep;
             a.use_changed = ph >= 4;
-            const int rows = g.members[m]->tile_rows;
+            const int rows = pmi::tile_rows(g.members[m], pmi::tile_warps(g.members[m]));  // one at a time
             const dim3 grid = pm::tile_grid(a.W, a.H, rows);
             pm::BandArgs band{};
             const pm::BandArgs *bp = nullptr;
-            const int rc = pmi::tile_band(g.members[m], grid, gs, &band, &bp);
+            const int rc = pmi::tile_band(g.members[m], rows, grid, gs, &band, &bp);
             if (rc) return rc;
             cudaError_t e = pm::dispatch_tile(g.S, g.kind, rows, grid, gs, a, bp);
             if (e != cudaSuccess) return fail(ctx, PM_ECUDA, "tile launch: %s", cudaGetErrorString(e));
@@ -544,6 +544,7 @@ int pm_batch_run(pm_batch *b) {
     PM_CUDA(ctx, cudaEventRecord(b->done, b->stream));
     for (pm_request *r : b->reqs) {
         PM_CUDA(ctx, cudaStreamWaitEvent(r->stream, b->done, 0));
+        pmi::note_running(r);
         r->postprocessed = r->prm.postprocess != 0;
     }
     ctx->launches += b->launches_per_run;

@@ -52,6 +52,7 @@ struct pm_ctx {
     size_t scratch_bytes = 0;
     int live = 0;  // requests, retained results and batches made from this context (cached included)
     int n_sm = 0;  // streaming multiprocessors: bands of the banded tile order
+    std::vector<pm_request *> running;  // requests whose last launches may still be on the device
 };
 
 struct pm_request {
@@ -59,8 +60,9 @@ struct pm_request {
     int W = 0, H = 0, S = 0;
     int batch_refs = 0;  // batches holding this request (it cannot be destroyed meanwhile)
     unsigned *band_ctr = nullptr;  // per-SM tile counters of the banded order (in the block)
-    int tile_rows = 8;             // tile height of its launches
-    int banded_blocks = 0;         // persistent grid of the banded order (0: one CTA per tile)
+    int tile_rows = 8;             // tile height of its next launches
+    long long company = 0;         // tile rows of the other requests in flight during its last run
+    int banded_blocks = 0;         // persistent grid of the banded order of large tiles (0: one CTA per tile)
     pm_params prm{};
     size_t bytes = 0;
     void *block = nullptr;  // one device allocation holding everything below
@@ -92,9 +94,14 @@ struct pm_request {
     pm::SweepArgs args{};
     cudaStream_t stream = nullptr;  // the request's own stream: requests overlap on the device
     cudaEvent_t ready = nullptr;    // recorded on this stream for requests seeded from it
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
-    bool graph_dirty = true;
+    // pm_request_run's launches, captured once per tile height
+    struct RunGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        bool current = false;  // captured since the views, parameters and seeds last changed
+    };
+    RunGraph small_run, large_run;
+    bool graph_dirty = true;  // neither is
     bool postprocessed = false;
 };
 
@@ -143,9 +150,12 @@ PM_INTERNAL int enqueue_post(pm_request *r, cudaStream_t st = nullptr);
 PM_INTERNAL long long tile_warps(const pm_request *r);
 PM_INTERNAL int tile_rows(const pm_request *r, long long warps);
 // The band arguments of the request's tile order for one launch of `grid`
-// on `st`, with the band counters reset there first; *out is null when the
+// with tiles of `rows` rows on `st`, with the band counters reset there first; *out is null when the
 // request runs one CTA per tile.
-PM_INTERNAL int tile_band(pm_request *r, dim3 grid, cudaStream_t st, pm::BandArgs *band, const pm::BandArgs **out);
+PM_INTERNAL int tile_band(pm_request *r, int rows, dim3 grid, cudaStream_t st, pm::BandArgs *band,
+                          const pm::BandArgs **out);
+// List the request among those that may be on the device.
+PM_INTERNAL void note_running(pm_request *r);
 // Enqueue r's seeding on st: landmark seeds, then its prior request or
 // retained result (the stage of pm_request_run between the init scoring and
 // the sweeps).  in_batch: the prior is a request of the same batch whose

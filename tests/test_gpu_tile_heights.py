@@ -28,3 +28,80 @@ def test_tile_heights_agree(ctx, W, H, S, sampler):
         assert all(np.array_equal(got[k].view(np.int32), alone[k].view(np.int32)) for k in want), executor
     b.close()
     r.close()
+
+
+@pytest.mark.parametrize("n_src", [2, 8])
+def test_height_follows_what_is_in_flight(ctx, n_src):
+    """Requests run without waiting for each other take large tiles once the
+    device is shared, and small ones again when they run alone: one after the
+    other, in flight together (in both orders), and alone again give the same
+    maps; a request destroyed with others in flight is no longer looked at."""
+    W, H, n = 320, 160, 8
+    want = ("depth", "score", "plane")
+    rs = []
+    for k in range(n):
+        req = scene.make_request(scene.ROOM_OBJECTS, W, H, n_src, seed=80 + k)
+        r = ctx.request(W, H, n_src, native.default_params(seed=k, iterations=3))
+        r.set_views([v.gray_u8 for v in req.views], req.R, req.t)
+        rs.append(r)
+    alone = []
+    for r in rs:
+        r.run()
+        alone.append(r.read(want=want))
+
+    def same(r, a):
+        got = r.read(want=want)
+        return all(np.array_equal(got[k].view(np.int32), a[k].view(np.int32)) for k in want)
+
+    for order in (range(n), range(n - 1, -1, -1)):
+        for k in order:
+            rs[k].run()
+        assert all(same(r, a) for r, a in zip(rs, alone))
+    for r in rs:
+        r.init()
+        r.sweep(0, 6)
+        r.postprocess()
+    assert all(same(r, a) for r, a in zip(rs, alone))
+    for r in rs:
+        r.run()
+    rs.pop().close()
+    rs[0].run()
+    assert all(same(r, a) for r, a in zip(rs, alone))
+    rs[0].synchronize()
+    rs[0].run()
+    assert same(rs[0], alone[0])
+    for r in rs:
+        r.close()
+
+
+def test_running_leaves_an_open_capture_alone(ctx):
+    """pm_request_run with other requests in flight, inside a capture that the
+    caller has open on another stream: the launches of a captured run are legal
+    there, and looking at what is in flight must stay so."""
+    import torch
+    rs = []
+    for k in range(3):
+        req = scene.make_request(scene.ROOM_OBJECTS, 192, 96, 2, seed=90 + k)
+        r = ctx.request(192, 96, 2, native.default_params(seed=k, iterations=2))
+        r.set_views([v.gray_u8 for v in req.views], req.R, req.t)
+        r.run()
+        r.synchronize()
+        rs.append(r)
+    for r in rs[:2]:  # the graph of either height
+        for q in rs:
+            q.run()
+        for q in rs:
+            q.synchronize()
+    want = rs[0].read(want=("depth",))["depth"]
+    x = torch.zeros(1000, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x += 1
+        rs[1].run()
+        rs[0].run()
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 1000.0
+    assert np.array_equal(rs[0].read(want=("depth",))["depth"], want)
+    for r in rs:
+        r.close()
