@@ -130,6 +130,8 @@ constexpr int kSmallWarpsTexture = 18, kSmallWarpsQuad = 12;
 // rows: 8 sources, textures u8 / FP16, 320x160 (8 rows either way) 1.03 / 1.04,
 // 384x192 (8) 1.05 / 1.07, 512x256 (16) 1.02 / 1.05, but 256x128 (4 for 8)
 // 0.85 / 0.86, 448x224 (12 for 16) 0.86 / 0.87, 576x288 (20 for 24) 0.99 / 0.96.
+// Exact samples of u8 images are even there (320x160 to 512x256 0.99 to 1.01, the
+// host variant 0.95 to 1.00) and keep small tiles.
 constexpr int kSmallBalanceSources = 8;
 // Tile rows per SM of the other requests in flight from which a small image runs
 // in large tiles too: n equal requests in flight, 8 sweeps, all in small against
@@ -246,7 +248,8 @@ int pmi::tile_rows(const pm_request *r, long long warps) {
     if (!few_tile_rows(r, warps)) return pm::kTileRowsLarge;
     // rows of the fullest SM with tiles of `rows` rows
     const auto fullest = [&](int rows) { return (warps + rows * n_sm - 1) / (rows * n_sm) * rows; };
-    if (r->S >= kSmallBalanceSources && fullest(pm::kTileRowsSmall) >= fullest(pm::kTileRowsLarge))
+    const bool byte_quads = r->prm.sampler == PM_SAMPLER_EXACT && r->prm.image_format == PM_IMAGE_U8;
+    if (r->S >= kSmallBalanceSources && !byte_quads && fullest(pm::kTileRowsSmall) >= fullest(pm::kTileRowsLarge))
         return pm::kTileRowsLarge;
     return pm::kTileRowsSmall;
 }
