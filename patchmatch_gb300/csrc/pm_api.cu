@@ -138,8 +138,10 @@ constexpr int kSmallBalanceSources = 8;
 // all in large tiles, textures, 2 / 4 / 6 / 8 sources (warps per SM of the others):
 // 2 of 512x256 (13) 0.92 / 1.00 / 0.98 / 1.00, 3 of 384x192 (15) 0.91 / 0.97 / 0.98 /
 // 1.06, 2 of 576x288 (17) 1.05 / 1.11 / 1.10 / 1.01, 3 of 448x224 (21) 1.09 / 1.15 /
-// 1.13 / 1.05, 8 of 256x128 (24) 1.06 / 1.11 / 1.32 / 1.48.
-constexpr int kSharedWarps = 16;
+// 1.13 / 1.05, 6 of 256x128 (17) 0.90 / 0.98 / 1.07 / 1.28, 8 of 256x128 (24) 1.06 /
+// 1.11 / 1.32 / 1.48.  Three in flight with 2 sweeps are up to 13 % slower in large
+// tiles at 18 to 19.  From 8 sources (kSmallBalanceSources) the line is lower.
+constexpr int kSharedWarps = 20, kSharedWarpsBalanced = 16;
 // Start alignment of the per-source sampling buffers: texture objects bound
 // to pitched linear memory need the device's texture alignment (512 bytes).
 constexpr size_t kTexAlign = 512;
@@ -271,8 +273,8 @@ static StreamState stream_state(const pm_request *q) {
 }
 
 // Choose the tile height of the request's next launches: large tiles when the
-// other requests of the context at work have kSharedWarps tile rows per SM, else
-// by its own size.  They are those on the device now or, if more, those that
+// other requests of the context at work have kSharedWarps (kSharedWarpsBalanced)
+// tile rows per SM, else by its own size.  They are those on the device now or, if more, those that
 // joined it during its last run: the first of a burst is alone when it is
 // enqueued.  1 / 2 / 4 / 8 / 12 requests of 384x192 with 4 sources in flight, 8
 // sweeps, every height by the request's own size: 2.55 / 3.52 / 6.62 / 13.3 / 19.8 ms,
@@ -280,7 +282,9 @@ static StreamState stream_state(const pm_request *q) {
 static void choose_tile_rows(pm_request *r) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(r->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
-    const long long own = pmi::tile_warps(r), shared = (long long)kSharedWarps * r->ctx->n_sm;
+    const int per_sm = r->S >= kSmallBalanceSources ? kSharedWarpsBalanced : kSharedWarps;
+    const long long own = pmi::tile_warps(r), shared = (long long)per_sm * r->ctx->n_sm;
+    const long long most = (long long)kSharedWarps * r->ctx->n_sm;
     std::vector<pm_request *> &run = r->ctx->running;
     std::vector<pm_request *> busy;
     long long others = 0;
@@ -290,7 +294,7 @@ static void choose_tile_rows(pm_request *r) {
     size_t kept = 0;
     for (pm_request *q : run) {
         if (q == r) continue;
-        if (others < shared || q->company < shared) {  // else the answer changes nothing
+        if (others < shared || q->company < most) {  // else the answer changes nothing
             const StreamState state = stream_state(q);
             if (state == StreamState::done) continue;
             if (state == StreamState::working) {
